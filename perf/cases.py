@@ -142,6 +142,17 @@ def _tokens(lead, nkvh, gen):
 
 
 def prepare(case, seed):
+    s = _state(case, seed)
+    if case.get("graph"):
+        _decode_layers(s)  # once before the capture: workspace and one-time set-up
+        torch.cuda.synchronize()
+        s["graph"] = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(s["graph"]):
+            _decode_layers(s)
+    return s
+
+
+def _state(case, seed):
     gen = _gen(seed)
     if case["kind"] == "batch":
         return _prepare_batch(case, gen)
@@ -166,12 +177,6 @@ def prepare(case, seed):
         outs["qn"] = layers[0]["qn"]
         outs["rows"] = [r for c in (layers[0]["kc"], layers[0]["vc"]) for r in _new_rows(c, nkvh, n_ctx, q8, n - T, n)]
     s["outs"] = outs
-    if case.get("graph"):
-        _decode_layers(s)  # once before the capture: workspace and one-time set-up
-        torch.cuda.synchronize()
-        s["graph"] = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(s["graph"]):
-            _decode_layers(s)
     return s
 
 
@@ -233,6 +238,88 @@ def run(s):
             if c["f16_qk"]:
                 q27.set_prefill_kernel(0)
     return s["outs"]
+
+
+def _norm_rope(x, w, pos):
+    """RMSNorm and rotary embedding of rows [token][head][256] at positions [token]; pairs (j, j + 32), j < 32."""
+    x = x.double()
+    x = x / (x.square().mean(-1, keepdim=True) + EPS).sqrt() * w.double()
+    theta = pos.double()[:, None, None] * THETA_SCALE ** torch.arange(32, dtype=torch.float64, device=x.device)
+    a, b = x[..., :32], x[..., 32:64]
+    return torch.cat([a * theta.cos() - b * theta.sin(), a * theta.sin() + b * theta.cos(), x[..., 64:]], -1)
+
+
+def _stored(x, q8):
+    """Rows as the cache gives them back: f16, or q8_0 with scales amax / 127 in f16 (and these scales)."""
+    if not q8:
+        return x.half().double(), None
+    b = x.reshape(*x.shape[:-1], 8, 32)
+    d = b.abs().amax(-1, keepdim=True) / 127.0
+    return (torch.round(b / d) * d.half().double()).reshape(x.shape), d[..., 0]
+
+
+def _attend(qn, qg, k, v, pos):
+    """One sequence: qn [T][nqh][256], k and v [nkvh][n][256] (the new rows included), pos [T]; the gated output."""
+    T, nkvh, n = qn.shape[0], k.shape[0], k.shape[1]
+    o = torch.empty((T, nkvh * GQA, AD), dtype=torch.float64, device=qn.device)
+    step = max(1, min(T, (1 << 28) // (GQA * n)))  # scores of at most 2 GB at a time
+    at = torch.arange(n, device=qn.device)
+    for h in range(nkvh):
+        for a in range(0, T, step):
+            q = qn[a:a + step, h * GQA:(h + 1) * GQA]
+            sc = (q.reshape(-1, AD) @ k[h].T).view(q.shape[0], GQA, n).mul_(KQ_SCALE)
+            sc.masked_fill_(at > pos[a:a + step, None, None], -math.inf)
+            o[a:a + step, h * GQA:(h + 1) * GQA] = (torch.softmax(sc, -1).view(-1, n) @ v[h]).view(q.shape)
+    return o * torch.sigmoid(qg[..., AD:].double())
+
+
+def _dequant(values, scales):
+    return (values.double().view(*values.shape[:-1], 8, 32) * scales.double()[..., None]).view(values.shape)
+
+
+def exact(case, seed):
+    """What run returns, in float64 from the same inputs (RoPE angles too). No value for whole numbers."""
+    s = _state(case, seed)
+    return _exact_batch(s) if case["kind"] == "batch" else _exact_one(s)
+
+
+def _exact_one(s):
+    T, nkvh, n_ctx, q8 = s["T"], s["nkvh"], s["n_ctx"], s["q8"]
+    first = int(s["pos"][0])
+    pos = torch.arange(first, first + T, device="cuda")
+    outs = {"result": []}
+    for w in s["layers"]:
+        qn, rows, kv = _norm_rope(w["qg"][..., :AD], w["q_norm"], pos), [], []
+        for c, x in ((w["kc"], _norm_rope(w["k"], w["k_norm"], pos)), (w["vc"], w["v"].double())):
+            x = x.transpose(0, 1)  # [nkvh][T][256], the cache's order
+            back, d = _stored(x, q8)
+            old = _dequant(*_parts(c, 1, nkvh, n_ctx))[0] if q8 else c.view(torch.float16).view(nkvh, n_ctx, AD).double()
+            old[:, first:first + T] = back
+            kv.append(old[:, :first + T])
+            rows += [None, d] if q8 else [x]
+        o = _attend(qn, w["qg"], *kv, pos)
+        if s["case"].get("q8_1"):
+            outs["result"] += [None, o.reshape(-1, 32).abs().amax(-1) / 127.0]
+        else:
+            outs["result"].append(o)
+        outs["qn"], outs["rows"] = qn, rows
+    return outs if len(s["layers"]) == 1 else {"result": outs["result"]}
+
+
+def _exact_batch(s):
+    B, T, nkvh = s["case"]["B"], s["case"]["T"], s["nkvh"]
+    pools = [_parts(s[which], s["n_pages"], nkvh, PAGE) for which in ("kpool", "vpool")]
+    o, qns = torch.empty(s["o"].shape, dtype=torch.float64, device="cuda"), torch.empty(s["qn"].shape, dtype=torch.float64, device="cuda")
+    for b, n in enumerate(s["lens"].tolist()):
+        pos = torch.arange(n - T, n, device="cuda")
+        qns[b] = _norm_rope(s["qg"][b][..., :AD], s["q_norm"], pos)
+        pg, kv = s["table"][b, :-(-n // PAGE)].long(), []
+        for (vals, scales), x in zip(pools, (_norm_rope(s["k"][b], s["k_norm"], pos), s["v"][b].double())):
+            whole = _dequant(vals[pg], scales[pg]).transpose(0, 1).reshape(nkvh, -1, AD)
+            whole[:, n - T:n] = _stored(x.transpose(0, 1), True)[0]
+            kv.append(whole[:, :n])
+        o[b] = _attend(qns[b], s["qg"][b], *kv, pos)
+    return {"kpool": [None, None], "vpool": [None, None], "o": o, "qn": qns}
 
 
 def work(case):
