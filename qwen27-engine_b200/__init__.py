@@ -28,7 +28,7 @@ OK, BAD_SHAPE, CUDA_ERROR, UNSUPPORTED, DEVICE_STATUS = 0, 1, 2, 3, 4
 SYMBOLS = [
     "q27b_last_error", "q27b_device_status", "q27b_kv_cache_bytes", "q27b_attn_chunks", "q27b_kv_append",
     "q27b_attn_prep", "q27b_attn_decode", "q27b_attn_decode_partial", "q27b_lse_merge", "q27b_attn_decode_paged",
-    "q27b_kv_pool_bytes", "q27b_attn_prefill", "q27b_prefill_qk_debug", "q27b_debug_split_event", "q27b_debug_split_events", "q27b_debug_split_only", "q27b_debug_decode_trace", "q27b_set_decode_kernel", "q27b_set_decode_schedule", "q27b_set_prefill_kernel", "q27b_prefill_split_plan", "q27b_sum_xbuf_bytes", "q27b_xbuf_alloc_bytes",
+    "q27b_kv_pool_bytes", "q27b_attn_prefill", "q27b_prefill_qk_debug", "q27b_debug_split_event", "q27b_debug_split_events", "q27b_debug_split_only", "q27b_debug_decode_trace", "q27b_set_decode_kernel", "q27b_set_decode_schedule", "q27b_set_prefill_kernel", "q27b_prefill_split_plan", "q27b_prefill_row_plan", "q27b_sum_xbuf_bytes", "q27b_xbuf_alloc_bytes",
     "q27b_sum_norm_q8", "q27b_sum_push", "q27b_sum_norm_q8_wait", "q27b_debug_expire_wait",
     "q27b_attn_prefill_q8_1", "q27b_xbuf_bytes", "q27b_attn_decode_partial_push", "q27b_lse_merge_wait",
     "q27b_xbuf_alloc", "q27b_xbuf_free", "q27b_ipc_export", "q27b_ipc_open", "q27b_ipc_close",
@@ -246,9 +246,18 @@ def set_decode_kernel(which):
     _check(_lib.q27b_set_decode_kernel(int(which)))
 
 
+def prefill_row_plan(M, nkvh, n_sm, depth_hint, must_merge=False):
+    """(split_tiles, pieces) of an attn_prefill call: of every KV head's ceil(6 M / 128) tiles of (token, head) rows the
+    first split_tiles are cut into `pieces` pieces over their positions, the others are not (host arithmetic only)."""
+    ts, ns = ctypes.c_int(0), ctypes.c_int(0)
+    _check(_lib.q27b_prefill_row_plan(int(M), int(nkvh), int(n_sm), int(depth_hint), int(bool(must_merge)), ctypes.byref(ts),
+                                      ctypes.byref(ns)))
+    return ts.value, ns.value
+
+
 def prefill_split_plan(M, nqh, n_sm, depth_hint):
-    """(split_tiles, pieces) of an attn_prefill call: the first split_tiles query tiles are cut into
-    `pieces` pieces over their positions, the others are not (host arithmetic only)."""
+    """The reference's rule for tiles of 128 tokens of one head: (split_tiles, pieces) (host arithmetic only;
+    attn_prefill plans with prefill_row_plan)."""
     ts, ns = ctypes.c_int(0), ctypes.c_int(0)
     _check(_lib.q27b_prefill_split_plan(int(M), int(nqh), int(n_sm), int(depth_hint), ctypes.byref(ts), ctypes.byref(ns)))
     return ts.value, ns.value

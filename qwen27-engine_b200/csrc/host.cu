@@ -102,12 +102,12 @@ int paged_ws(DeviceCtx* ctx, size_t floats, float** out) {
   return Q27B_OK;
 }
 
-int fit_prefill_split(DeviceCtx* ctx, int* ts, int* ns, int M, int nqh, bool must_merge, float** part) {
+int fit_prefill_split(DeviceCtx* ctx, int* ts, int* ns, int tokens, int nqh, bool must_merge, float** part) {
   *part = nullptr;
   if (*ns <= 1) return Q27B_OK;
   size_t cap = 0;
   if (int rc = prefill_ws(ctx, part, &cap)) return rc;
-  const size_t per_piece = (size_t)std::min(M, *ts * 128) * nqh * PROW;
+  const size_t per_piece = (size_t)tokens * nqh * PROW;
   const int fit = (int)std::min<size_t>(64, cap / per_piece);
   if (*ns > fit) *ns = fit;
   if (*ns < 2) {

@@ -61,10 +61,9 @@ int prefill_ws(DeviceCtx* ctx, float** out, size_t* max_floats);
 // The batched-decode partial buffer with room for `floats`; grows (free + allocate) when it has to,
 // unless the workspace is frozen, in which case a larger request fails with Q27B_UNSUPPORTED.
 int paged_ws(DeviceCtx* ctx, size_t floats, float** out);
-// Cuts a prefill split plan (ts tiles cut into ns pieces, partial rows Ms * nqh) to what the prefill
-// buffer holds: fewer pieces, or no split at all; must_merge (q8_1 through the merge kernel) fails
+// Cuts a prefill split plan (ts tiles, `tokens` tokens, cut into ns pieces) to what the prefill buffer holds: fewer pieces, or no split at all; must_merge (q8_1 through the merge kernel) fails
 // instead when not even two pieces fit.
-int fit_prefill_split(DeviceCtx* ctx, int* ts, int* ns, int M, int nqh, bool must_merge, float** part);
+int fit_prefill_split(DeviceCtx* ctx, int* ts, int* ns, int tokens, int nqh, bool must_merge, float** part);
 
 // True when Q27_PDL=1, the reference's switch with the reference's default (off; src/ops.cu:12-15,
 // src/common.cuh:28-42): kernels are then launched with the programmatic-stream-serialization

@@ -9,8 +9,11 @@
 // no max offset is needed; the reference max of a row is only moved when its true max has grown
 // by more than TAU, which keeps P <= e^TAU and makes the O rescale rare.
 //
-// One CTA = 128 query tokens of one query head (TMEM lane = token) x one split of the positions,
-// walking 64-position tiles. Roles (14 warps):
+// One CTA = 128 rows of one KV head (TMEM lane = row) x one split of the positions, walking 64-position
+// tiles. The rows of a KV head are its M * 6 (token, head) pairs, token-major: a tile spans 22 tokens of all
+// six heads, so that only the last tile of a KV head has empty rows (tiles of 128 tokens of one head: 16 tokens
+// behind 30,000 took 293 us, now 64; 131 behind 30,011 521, now 274) and fewer position tiles are half masked.
+// Roles (14 warps):
 //   warps 0-7   softmax, two warpgroups: both own the 128 rows (warp w and w+4 share TMEM lanes
 //               32(w%4)..), warpgroup 0 takes positions 0-31 of a tile, warpgroup 1 positions
 //               32-63. Each thread reads its half of the per-block int32 accumulators from TMEM,
@@ -34,7 +37,7 @@
 namespace q27b {
 namespace {
 
-constexpr int QT = 128;          // query tokens per CTA
+constexpr int QT = 128;          // query rows per CTA
 constexpr int PT = 64;           // positions per tile
 constexpr float TAU = 5.0f;      // the reference max moves only when the true max exceeds it by this much
 
@@ -99,11 +102,12 @@ struct PrefillParams {
   const float* qn;   // [M][nqh][256]
   const float* qg;   // [M][nqh][512]
   float* o;          // [M][nqh][256]
-  float* part;       // [nsplit][Ms][nqh][258], Ms = min(M, 128 ts): the tokens whose positions are split
+  float* part;       // [nsplit][Ms][nqh][258]
   const int* pos0;
   int* status;
   int M, nqh, nkvh, n_ctx;
-  int ts, nsplit;    // query tiles [0, ts) are split nsplit ways over their positions, the others are not
+  int Ms;            // tokens of the split tiles
+  int ts, nsplit;    // row tiles [0, ts) are split nsplit ways over their positions, the others are not
   float kq_scale;
   int tile_major;  // CTA order, see the kernel
   int8_t* xq;      // q8_1 output instead of o: int8 [M][nqh][256] ...
@@ -192,34 +196,35 @@ prefill_i8_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_consta
   volatile int* abort_flag = (volatile int*)(sgen + OFF_MISC + 4);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // CTA order: the query tiles with the most positions first (src/attn.cu:567). tile_major: and that
-  // across all heads (block L = head L % nqh of tile rank L / nqh), which matters on a short prefix,
+  // CTA order: the row tiles with the most positions first (src/attn.cu:567). tile_major: and that
+  // across all KV heads (block L = KV head L % nkvh of tile rank L / nkvh), which matters on a short prefix,
   // where the tiles differ a lot in length and the longest tiles of the last heads would start last.
-  // Otherwise head by head (block L = tile rank L % n_tiles of head L / n_tiles), so that the CTAs
+  // Otherwise KV head by KV head (block L = tile rank L % n_tiles of KV head L / n_tiles), so that the CTAs
   // that run at the same time stream the same K/V rows and share them in L2 (measured: 7 % at 32k).
   // The unsplit CTAs (tiles >= ts) come first, then the pieces of the split tiles, split index slowest.
-  int L = (int)blockIdx.x, z = 0, nsplit = 1, ntl = (p.M + QT - 1) / QT - p.ts, tile_base = p.ts;
-  if (L >= ntl * p.nqh) {
-    L -= ntl * p.nqh;
+  int L = (int)blockIdx.x, z = 0, nsplit = 1, ntl = row_tiles(p.M) - p.ts, tile_base = p.ts;
+  if (L >= ntl * p.nkvh) {
+    L -= ntl * p.nkvh;
     ntl = p.ts;
     tile_base = 0;
     nsplit = p.nsplit;
-    z = L / (ntl * p.nqh);
-    L -= z * ntl * p.nqh;
+    z = L / (ntl * p.nkvh);
+    L -= z * ntl * p.nkvh;
   }
-  const int h = p.tile_major ? L % p.nqh : L / ntl, kh = h / GQA;
-  const int t0 = (tile_base + ntl - 1 - (p.tile_major ? L / p.nqh : L % ntl)) * QT;
-  const int Ms = min(p.M, p.ts * QT);
+  const int kh = p.tile_major ? L % p.nkvh : L / ntl;
+  const int row0 = (tile_base + ntl - 1 - (p.tile_major ? L / p.nkvh : L % ntl)) * QT;  // first row of this CTA
+  const int t0 = row0 / GQA;                                                            // and its token
   const int pos0 = *p.pos0;
-  const int n_end = min(pos0 + min(t0 + QT, p.M), p.n_ctx);
+  const int n_end = min(pos0 + min((row0 + QT - 1) / GQA + 1, p.M), p.n_ctx);
   const int ntot = (n_end + PT - 1) / PT;
   const int per = (ntot + nsplit - 1) / nsplit;
   const int it0 = min(ntot, z * per), it1 = min(ntot, it0 + per);
   const int nt = it1 - it0;
 
   if (nt <= 0) {  // nothing in this split: neutral partials
-    if (nsplit > 1 && tid < QT && t0 + tid < p.M) {
-      float* po = p.part + (((size_t)z * Ms + t0 + tid) * p.nqh + h) * PROW;
+    const int t = (row0 + tid) / GQA, h = kh * GQA + (row0 + tid) % GQA;
+    if (nsplit > 1 && tid < QT && t < p.M) {
+      float* po = p.part + (((size_t)z * p.Ms + t) * p.nqh + h) * PROW;
       po[0] = M_INIT;
       po[1] = 0.f;
       for (int d = 0; d < AD; d++) po[2 + d] = 0.f;
@@ -261,7 +266,7 @@ prefill_i8_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_consta
     // ================================================================ softmax warps
     const int wg = warp >> 2, q = warp & 3;
     const int r = q * 32 + lane;       // query row = TMEM lane
-    const int t = t0 + r;
+    const int t = (row0 + r) / GQA, h = kh * GQA + (row0 + r) % GQA;
     const bool live = t < p.M;
     float* xch = (float*)(sgen + OFF_XCH);
     const float* dqs = (const float*)(sgen + OFF_DQ) + r;  // block b of this row at dqs[b * QT]
@@ -418,7 +423,7 @@ prefill_i8_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_consta
     mbar_wait(&bar[B_ODONE], 0, abort_flag, p.status);
     tc_fence_after();
     const float inv_l = 1.0f / l;
-    float* po = nsplit > 1 ? p.part + (((size_t)z * Ms + t) * p.nqh + h) * PROW : nullptr;
+    float* po = nsplit > 1 ? p.part + (((size_t)z * p.Ms + t) * p.nqh + h) * PROW : nullptr;
     if (live && po && wg == 0) {
       po[0] = m_ref;
       po[1] = l;
@@ -754,6 +759,14 @@ int q27b_prefill_split_plan(int M, int nqh, int n_sm, int depth_hint, int* split
   return Q27B_OK;
 }
 
+int q27b_prefill_row_plan(int M, int nkvh, int n_sm, int depth_hint, int must_merge, int* split_tiles, int* pieces) {
+  if (M < 1 || nkvh < 1 || n_sm < 1 || !split_tiles || !pieces) return fail(Q27B_BAD_SHAPE, "prefill_row_plan: bad argument");
+  const SplitPlan sp = plan_prefill_rows(M, nkvh, n_sm, depth_hint, must_merge != 0);
+  *split_tiles = sp.ts;
+  *pieces = sp.ns;
+  return Q27B_OK;
+}
+
 int q27b_set_prefill_kernel(int which) {
   if (which < 0 || which > 2) return fail(Q27B_BAD_SHAPE, "set_prefill_kernel: 0 auto, 1 int8 QK, 2 f16 QK");
   g_prefill_choice.store(which);
@@ -773,20 +786,20 @@ static int prefill_impl(const float* qn, const float* qg, const void* kcache, co
                               depth_hint, (cudaStream_t)stream);
   if (int rc = prefill_setup(ctx)) return rc;
   cudaStream_t s = (cudaStream_t)stream;
-  const int tiles = (M + QT - 1) / QT;
-  SplitPlan sp = plan_prefill_split(tiles, nqh, ctx->n_sm, M, depth_hint, false);
+  const int tiles = row_tiles(M);
+  SplitPlan sp = plan_prefill_rows(M, nkvh, ctx->n_sm, depth_hint, false);
   float* part;  // the fixed prefill workspace; the plan is cut to what it holds
-  if (int rc = fit_prefill_split(ctx, &sp.ts, &sp.ns, M, nqh, false, &part)) return rc;
-  const int nsplit = sp.ns, Ms = std::min(M, sp.ts * QT);
+  if (int rc = fit_prefill_split(ctx, &sp.ts, &sp.ns, split_tokens(M, sp.ts), nqh, false, &part)) return rc;
+  const int nsplit = sp.ns, Ms = split_tokens(M, sp.ts);
   CUtensorMap kvm, ksm, vvm, vsm;
   if (int rc = q8_tmaps(kcache, (uint64_t)nkvh * n_ctx, &kvm, &ksm)) return rc;
   if (int rc = q8_tmaps(vcache, (uint64_t)nkvh * n_ctx, &vvm, &vsm)) return rc;
   const CUtensorMap *kv = &kvm, *ks = &ksm, *vv = &vvm, *vs = &vsm;
   PrefillParams p = {};
   p.qn = qn; p.qg = qg; p.o = o; p.xq = xq; p.xd = xd; p.part = nsplit > 1 ? part : nullptr; p.pos0 = pos0; p.status = ctx->status;
-  p.M = M; p.nqh = nqh; p.nkvh = nkvh; p.n_ctx = n_ctx; p.ts = sp.ts; p.nsplit = nsplit; p.kq_scale = kq_scale;
+  p.M = M; p.nqh = nqh; p.nkvh = nkvh; p.n_ctx = n_ctx; p.Ms = Ms; p.ts = sp.ts; p.nsplit = nsplit; p.kq_scale = kq_scale;
   p.tile_major = depth_hint >= 0 && depth_hint < 4 * M;  // short prefix: the causal part dominates
-  prefill_i8_kernel<<<(tiles - sp.ts) * nqh + sp.ts * nqh * nsplit, PF_THREADS, PF_SMEM_BYTES, s>>>(*kv, *ks, *vv, *vs, p);
+  prefill_i8_kernel<<<(tiles - sp.ts) * nkvh + sp.ts * nkvh * nsplit, PF_THREADS, PF_SMEM_BYTES, s>>>(*kv, *ks, *vv, *vs, p);
   Q27B_CK(cudaGetLastError());
   if (nsplit > 1) {  // the split tokens are rows [0, Ms * nqh) of every array
     MergeParams mp = {};

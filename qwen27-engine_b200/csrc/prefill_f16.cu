@@ -9,7 +9,7 @@
 // K-major for K, read MN-major for V; ring of three stages each): no converter warps, no per-block
 // scale arithmetic.
 //
-// One CTA = 128 query tokens of one query head (TMEM lane = token) x one split of the positions.
+// One CTA = 128 (token, head) rows of one KV head (TMEM lane = row; see prefill.cu) x one split of the positions.
 // Warps 0-7 softmax (two warpgroups, 32 columns of a tile each), warp 8 TMA producer, warp 9 issues
 // the Q K^T MMAs (per tile 16 x (128x64x16) into one of two S buffers), warp 10 the P V MMAs
 // (4 x (128x256x16) into O).
@@ -33,7 +33,7 @@
 namespace q27b {
 namespace {
 
-constexpr int QT = 128;          // query tokens per CTA
+constexpr int QT = 128;          // query rows per CTA
 constexpr int PT = 64;           // positions per tile
 constexpr float TAU = 5.0f;
 constexpr int SEGK = PT * 128;   // one 64-dim segment of a K or V tile: [64 positions][128 B]
@@ -77,12 +77,14 @@ struct F16Params {
   const float* qn;   // [M][nqh][256]
   const float* qg;   // [M][nqh][512]
   float* o;          // [M][nqh][256]
-  float* part;       // [nsplit][Ms][nqh][258], Ms = min(M, 128 ts): the tokens whose positions are split
+  float* part;       // [nsplit][Ms][nqh][258]
   const int* pos0;
   int* status;
   int M, nqh, nkvh, n_ctx;
-  int ts, nsplit;    // query tiles [0, ts) are split nsplit ways over their positions, the others are not
+  int Ms;            // tokens of the split tiles
+  int ts, nsplit;    // row tiles [0, ts) are split nsplit ways over their positions, the others are not
   float kq_scale;
+  int tile_major;    // CTA order: tile by tile across the KV heads instead of head by head
 };
 
 // the NWG threads of a query row sit in warp q of every softmax warpgroup
@@ -179,30 +181,31 @@ prefill_f16_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // CTA order: the unsplit CTAs (tiles >= ts) first, then the pieces of the split tiles, split index
-  // slowest; within each class head by head, the query tiles with the most positions first
-  // (src/attn.cu:567)
-  int L = (int)blockIdx.x, z = 0, nsplit = 1, ntl = (p.M + QT - 1) / QT - p.ts, tile_base = p.ts;
-  if (L >= ntl * p.nqh) {
-    L -= ntl * p.nqh;
+  // slowest; within each class KV head by KV head (on a short prefix, where the tiles differ in length,
+  // tile by tile across the KV heads), the row tiles with the most positions first (src/attn.cu:567)
+  int L = (int)blockIdx.x, z = 0, nsplit = 1, ntl = row_tiles(p.M) - p.ts, tile_base = p.ts;
+  if (L >= ntl * p.nkvh) {
+    L -= ntl * p.nkvh;
     ntl = p.ts;
     tile_base = 0;
     nsplit = p.nsplit;
-    z = L / (ntl * p.nqh);
-    L -= z * ntl * p.nqh;
+    z = L / (ntl * p.nkvh);
+    L -= z * ntl * p.nkvh;
   }
-  const int h = L / ntl, kh = h / GQA;
-  const int t0 = (tile_base + ntl - 1 - L % ntl) * QT;
-  const int Ms = min(p.M, p.ts * QT);
+  const int kh = p.tile_major ? L % p.nkvh : L / ntl;
+  const int row0 = (tile_base + ntl - 1 - (p.tile_major ? L / p.nkvh : L % ntl)) * QT;  // first row of this CTA
+  const int t0 = row0 / GQA;                                                            // and its token
   const int pos0 = *p.pos0;
-  const int n_end = min(pos0 + min(t0 + QT, p.M), p.n_ctx);
+  const int n_end = min(pos0 + min((row0 + QT - 1) / GQA + 1, p.M), p.n_ctx);
   const int ntot = (n_end + PT - 1) / PT;
   const int per = (ntot + nsplit - 1) / nsplit;
   const int it0 = min(ntot, z * per), it1 = min(ntot, it0 + per);
   const int nt = it1 - it0;
 
   if (nt <= 0) {  // nothing in this split: neutral partials
-    if (nsplit > 1 && tid < QT && t0 + tid < p.M) {
-      float* po = p.part + (((size_t)z * Ms + t0 + tid) * p.nqh + h) * PROW;
+    const int t = (row0 + tid) / GQA, h = kh * GQA + (row0 + tid) % GQA;
+    if (nsplit > 1 && tid < QT && t < p.M) {
+      float* po = p.part + (((size_t)z * p.Ms + t) * p.nqh + h) * PROW;
       po[0] = M_INIT;
       po[1] = 0.f;
       for (int d = 0; d < AD; d++) po[2 + d] = 0.f;
@@ -245,7 +248,7 @@ prefill_f16_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     // ================================================================ softmax warps
     const int wg = warp >> 2, q = warp & 3;
     const int r = q * 32 + lane;       // query row = TMEM lane
-    const int t = t0 + r;
+    const int t = (row0 + r) / GQA, h = kh * GQA + (row0 + r) % GQA;
     const bool live = t < p.M;
     float* xch = (float*)(sgen + OFF_XCH);
     const uint32_t tlane = tmem + ((uint32_t)(q * 32) << 16);
@@ -385,7 +388,7 @@ prefill_f16_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     mbar_wait(&bar[B_ODONE], 0, abort_flag, p.status);
     tc_fence_after();
     const float inv_l = 1.0f / l;
-    float* po = nsplit > 1 ? p.part + (((size_t)z * Ms + t) * p.nqh + h) * PROW : nullptr;
+    float* po = nsplit > 1 ? p.part + (((size_t)z * p.Ms + t) * p.nqh + h) * PROW : nullptr;
     if (live && po && wg == 0) {
       po[0] = m_ref;
       po[1] = l;
@@ -554,13 +557,13 @@ int launch_prefill_f16(DeviceCtx* ctx, const float* qn, const float* qg, const v
     attr[ctx->dev] = true;
   }
   static const int nwg_f16 = [] { const char* e = getenv("Q27B_PF16_NWG"); return e && e[0] == '4' ? 4 : 2; }();
-  const int tiles = (M + QT - 1) / QT;
+  const int tiles = row_tiles(M);
   // splits over the positions as for the int8 kernel; the q8_1 output is written by the merge kernel,
   // so it needs every tile on the split path (at least one merge)
-  SplitPlan sp = plan_prefill_split(tiles, nqh, ctx->n_sm, M, depth_hint, xq != nullptr);
+  SplitPlan sp = plan_prefill_rows(M, nkvh, ctx->n_sm, depth_hint, xq != nullptr);
   float* part;  // the fixed prefill workspace; the plan is cut to what it holds
-  if (int rc = fit_prefill_split(ctx, &sp.ts, &sp.ns, M, nqh, xq != nullptr, &part)) return rc;
-  const int nsplit = sp.ns, Ms = std::min(M, sp.ts * QT);
+  if (int rc = fit_prefill_split(ctx, &sp.ts, &sp.ns, split_tokens(M, sp.ts), nqh, xq != nullptr, &part)) return rc;
+  const int nsplit = sp.ns, Ms = split_tokens(M, sp.ts);
   CUtensorMap tkm, tvm, tksm, tvsm;
   const uint64_t rows = (uint64_t)nkvh * n_ctx;
   if (q8) {
@@ -576,8 +579,9 @@ int launch_prefill_f16(DeviceCtx* ctx, const float* qn, const float* qg, const v
   const CUtensorMap *tk = &tkm, *tv = &tvm, *tks = &tksm, *tvs = &tvsm;
   F16Params p = {};
   p.qn = qn; p.qg = qg; p.o = o; p.part = nsplit > 1 ? part : nullptr; p.pos0 = pos0; p.status = ctx->status;
-  p.M = M; p.nqh = nqh; p.nkvh = nkvh; p.n_ctx = n_ctx; p.ts = sp.ts; p.nsplit = nsplit; p.kq_scale = kq_scale;
-  const int grid = (tiles - sp.ts) * nqh + sp.ts * nqh * nsplit;
+  p.M = M; p.nqh = nqh; p.nkvh = nkvh; p.n_ctx = n_ctx; p.Ms = Ms; p.ts = sp.ts; p.nsplit = nsplit; p.kq_scale = kq_scale;
+  p.tile_major = depth_hint >= 0 && depth_hint < 4 * M;  // short prefix: the causal part dominates
+  const int grid = (tiles - sp.ts) * nkvh + sp.ts * nkvh * nsplit;
   if (q8)
     prefill_f16_kernel<true, 2><<<grid, Lay<true, 2>::THREADS, Lay<true, 2>::SMEM_BYTES, s>>>(*tk, *tv, *tks, *tvs, p);
   else if (nwg_f16 == 4)

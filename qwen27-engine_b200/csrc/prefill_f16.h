@@ -4,22 +4,25 @@
 #include "host.h"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 
 namespace q27b {
 
-// How the CTAs of a prefill call (one per 128-token query tile and head, one CTA per SM at a time)
-// split their positions. Tiles [0, ts) are split ns ways (partials + merge), tiles >= ts are not.
+// How the CTAs of a prefill call (one CTA per SM at a time) split their positions: tiles [0, ts) are split ns ways
+// (partials + merge), tiles >= ts are not.
+struct SplitPlan {
+  int ts, ns;
+};
+// The reference's rule for tiles of 128 tokens of one head, and a tail split of the same tiles (q27b_prefill_split_plan;
+// the launchers plan with plan_prefill_rows).
 //  * Few CTAs: every tile is split, enough CTAs for every SM and at least 2048 positions per split
-//    (the reference's rule, src/attn.cu:945-951). Q27_ATTN_SPLIT forces this form (src/attn.cu:952).
+//    (src/attn.cu:945-951). Q27_ATTN_SPLIT forces this form (src/attn.cu:952).
 //  * More CTAs than SMs on a deep prefix (all CTAs about equally long): the CTAs beyond the last full
 //    wave would leave most SMs idle for a whole CTA time (384 CTAs on 148 SMs: 3 rounds for 2.6
 //    rounds of work). The unsplit CTAs are launched first and only the earliest ts tiles - as many
 //    CTAs as the remainder - are cut into ns pieces that fill the machine evenly at the end; ns is
 //    the count that minimises the modelled makespan. Only ts / tiles of the rows pay for a merge.
-struct SplitPlan {
-  int ts, ns;
-};
 inline SplitPlan plan_prefill_split(int tiles, int nqh, int n_sm, int M, int depth_hint, bool must_merge) {
   const int ctas = tiles * nqh;
   int ns = 1;
@@ -46,6 +49,62 @@ inline SplitPlan plan_prefill_split(int tiles, int nqh, int n_sm, int M, int dep
   }
   if (tail && atoi(tail) > 1) best_ns = std::min(atoi(tail), ns_max);  // tuning: Q27B_PREFILL_TAIL_SPLIT=<pieces>
   return best_ns > 1 ? SplitPlan{ts, best_ns} : SplitPlan{0, 1};
+}
+
+// The query rows of a KV head are its M * 6 (token, head) pairs, token-major; a CTA takes 128 of them.
+constexpr int PF_ROWS = 128, PF_GQA = 6;
+__host__ __device__ inline int row_tiles(int M) { return (int)(((int64_t)M * PF_GQA + PF_ROWS - 1) / PF_ROWS); }
+// Tokens of the first ts row tiles. Three tiles are 64 tokens; a plan that splits some tiles and not others cuts there.
+inline int split_tokens(int M, int ts) { return ts >= row_tiles(M) ? M : ts / 3 * 64; }
+
+// The plan of a prefill call: the first ts row tiles of every KV head are cut into ns pieces over their positions.
+// A model of the launch in units of one 64-position tile of a CTA (one CTA per SM at a time): a CTA costs its tiles and
+// C0 more (Q tile, pipeline fill, epilogue), a piece CP on top of that (its partials are written), a merge M0 (launch)
+// and MROW + MPART * pieces for each row. Three forms compete:
+//  * nothing is split;
+//  * every tile is split. Few rows behind a long prefix leave most SMs idle otherwise, and a second, partly filled
+//    round of CTAs costs as much as a full one: 131 tokens behind 30,011 are 28 tiles, 5 pieces each fill one round of
+//    148 SMs (274 us; 3 pieces 407, 10 pieces 293). The other end: 1,000 tokens of one KV head behind 100, 47 tiles of
+//    17 position tiles, 55 us unsplit and 85 in 3 pieces: the merge of 6,000 rows costs more than the idle SMs.
+//  * tail split: more CTAs than SMs on a deep prefix. The unsplit CTAs are launched first; only the earliest ts tiles,
+//    as many CTAs as the last round would hold, are cut, and their pieces fill the machine evenly at the end. 2048
+//    tokens behind 32,768 / 148,000: 3,640 / 15,611 us unsplit, 3,363 / 13,741 with 5 pieces, 3,386 / 13,854 with 8.
+// On a short prefix the tiles differ in length (the causal part): longest first, no split once there is a CTA per SM.
+inline SplitPlan plan_prefill_rows(int M, int nkvh, int n_sm, int depth_hint, bool must_merge) {
+  constexpr double C0 = 3.0, CP = 4.0, M0 = 2.0, MROW = 1.2e-3, MPART = 2.0e-4;
+  const int rt = row_tiles(M), ctas = rt * nkvh;
+  if (const char* e = getenv("Q27_ATTN_SPLIT")) {
+    const int f = atoi(e);
+    if (f > 0) return {f > 1 || must_merge ? rt : 0, std::max(std::min(f, 64), must_merge ? 2 : 1)};
+  }
+  if (depth_hint < 0) return must_merge ? SplitPlan{rt, 2} : SplitPlan{0, 1};
+  const bool deep = depth_hint >= M;
+  if (!must_merge && !deep && ctas > n_sm) return {0, 1};
+  const double N = ((double)depth_hint + M) / 64, rows = (double)M * nkvh * PF_GQA;
+  const int ns_max = std::max(2, std::min(64, (int)(N / 2)));  // two position tiles a piece at least
+  auto rounds = [&](double n) { return std::ceil(n / n_sm - 1e-9); };
+  SplitPlan plan = must_merge ? SplitPlan{rt, 2} : SplitPlan{0, 1};
+  double best = must_merge ? 1e300 : rounds(ctas) * (N + C0);
+  for (int k = 2; k <= ns_max && (k == 2 || (int64_t)ctas * (k - 1) < 4 * n_sm); k++) {
+    const double t = rounds((double)ctas * k) * (N / k + C0 + CP) + M0 + rows * (MROW + MPART * k);
+    if (t < best) best = t, plan = {rt, k};
+  }
+  const char* tail = getenv("Q27B_PREFILL_TAIL_SPLIT");
+  if (must_merge || (tail && tail[0] == '0') || ctas <= n_sm || ctas % n_sm == 0) return plan;
+  const int ts = ((ctas % n_sm + nkvh - 1) / nkvh + 2) / 3 * 3;  // whole tokens: see split_tokens
+  if (ts >= rt) return plan;
+  const int U = ctas - ts * nkvh, b = U % n_sm;
+  const int forced = tail ? std::min({atoi(tail), ns_max, 8}) : 0;  // tuning: Q27B_PREFILL_TAIL_SPLIT=<pieces>
+  for (int k = 2; k <= std::min(ns_max, 8); k++) {
+    const double piece = N / k + C0 + CP;
+    // pieces that run beside the last, partly filled round of unsplit CTAs; a tenth of a round more than a whole
+    // number does not start another one (the unsplit CTAs do not end all at once)
+    const double left = std::max(0.0, (double)ts * nkvh * k - (b ? (n_sm - b) * std::floor((N + C0) / piece) : 0.0));
+    const double t = rounds(U) * (N + C0) + rounds(std::max(0.0, left - 0.1 * n_sm)) * piece + M0 +
+                     rows * split_tokens(M, ts) / M * (MROW + MPART * k);
+    if (forced > 1 ? k == forced : t < best) best = t, plan = {ts, k};
+  }
+  return plan;
 }
 
 // The f16-QK kernel: on an f16 cache (q8 = false), or on a q8_0 cache whose K and V it dequantises to

@@ -99,6 +99,30 @@ def test_prefill_split_plan(q27, monkeypatch):
     assert q27.prefill_split_plan(2048, 24, 148, 32768) == (0, 1)
 
 
+def test_prefill_row_plan(q27, monkeypatch):
+    """Host arithmetic of the plan over (token, head) rows: a plan that splits some tiles and not others cuts
+    between tokens (three tiles are 64 tokens), no piece is shorter than two position tiles, and without a depth
+    hint nothing is split unless the merge has to write the output."""
+    monkeypatch.delenv("Q27_ATTN_SPLIT", raising=False)
+    monkeypatch.delenv("Q27B_PREFILL_TAIL_SPLIT", raising=False)
+    for M in (1, 16, 21, 22, 43, 64, 85, 128, 131, 500, 1537, 2048, 4096):
+        tiles = (6 * M + 127) // 128
+        for nkvh in (1, 2, 4):
+            assert q27.prefill_row_plan(M, nkvh, 148, -1) == (0, 1)
+            assert q27.prefill_row_plan(M, nkvh, 148, -1, True) == (tiles, 2)
+            for depth in (0, 100, 5000, 30011, 148000):
+                ts, ns = q27.prefill_row_plan(M, nkvh, 148, depth)
+                assert (ts == 0) == (ns == 1) and 1 <= ns <= 64
+                assert ts in (0, tiles) or (ts % 3 == 0 and 0 < ts < tiles)
+                assert ns == 1 or ns * 128 <= depth + M or ns == 2
+                assert q27.prefill_row_plan(M, nkvh, 148, depth, True)[0] == tiles
+    # few rows on a deep prefix: the pieces of one round of the SMs
+    ts, ns = q27.prefill_row_plan(16, 4, 148, 30000)
+    assert ts == 1 and 4 * ns <= 148 and ns >= 20
+    monkeypatch.setenv("Q27_ATTN_SPLIT", "3")
+    assert q27.prefill_row_plan(2048, 4, 148, 32768) == (96, 3)
+
+
 def test_sum_norm_entry_points_check_their_arguments(q27):
     """Argument checks of the sum_norm family come before any CUDA call."""
     lib = ctypes.CDLL(q27.LIB_PATH)

@@ -66,6 +66,38 @@ def test_prefill_matches_oracle(q27, orc, pos0, M, nkvh):
     assert q27.device_status() == 0
 
 
+@pytest.mark.parametrize("M", [1, 21, 22, 43, 64, 85, 128, 150])
+@pytest.mark.parametrize("kernel", ["i8", "f16qk", "f16"])
+def test_prefill_row_tiles(q27, orc, M, kernel):
+    """Tiles of 128 (token, head) rows at their edges: 21 tokens leave two rows of a tile, 22 open the second, 64 fill
+    three; unsplit and cut into pieces."""
+    nkvh, pos0 = 2, 700
+    nqh = nkvh * GQA
+    qn, qg, kc_ref, vc_ref, n, n_ctx = make_case(orc, M, pos0, nkvh)
+    q8 = kernel != "f16"
+    if q8:
+        kc, vc = poisoned_cache(q27, kc_ref, nkvh, n_ctx, n), poisoned_cache(q27, vc_ref, nkvh, n_ctx, n)
+    else:
+        from qwen27_engine_b200 import synth
+        kc_ref, vc_ref = orc.fill_cache(synth.normal(synth.SEED_K, (nkvh, n, AD)), synth.normal(synth.SEED_V, (nkvh, n, AD)),
+                                        n_ctx, q8=False)
+        kc, vc = poisoned_cache(q27, kc_ref, nkvh, n_ctx, n, False), poisoned_cache(q27, vc_ref, nkvh, n_ctx, n, False)
+    if kernel == "i8":
+        ref = orc.attn_prefill_i8(qn, qg, kc_ref, vc_ref, pos0, SCALE, nkvh, n_ctx)
+    else:
+        ref = orc.attn_ref(qn, qg, kc_ref, vc_ref, pos0, SCALE, nkvh, n_ctx, q8=q8)
+    q27.set_prefill_kernel(2 if kernel == "f16qk" else 0)
+    try:
+        for depth_hint in (-1, pos0):
+            o = torch.full((M, nqh, AD), float("nan"), device="cuda")
+            q27.attn_prefill(dev(qn), dev(qg), kc, vc, o, pos_tensor(pos0), M, SCALE, nqh, nkvh, n_ctx, q8, depth_hint)
+            torch.cuda.synchronize()
+            assert_close(o.cpu().numpy(), ref, "%s M=%d depth_hint=%d" % (kernel, M, depth_hint))
+    finally:
+        q27.set_prefill_kernel(0)
+    assert q27.device_status() == 0
+
+
 @pytest.mark.parametrize("depth_hint", [8000, -1])
 def test_prefill_split_kv(q27, orc, depth_hint):
     """With a depth hint the positions are split over CTAs and merged by log-sum-exp."""
