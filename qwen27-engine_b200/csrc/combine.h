@@ -29,6 +29,11 @@ struct MergeParams {
   int* xbuf;            // this rank's own exchange buffer (push: epoch and counter; wait: everything)
   int wait_n;
   int* status;
+  // Decode layout, one sequence (null otherwise): the split-K kernel leaves the partials of chunks without a tile
+  // unwritten when no chunk has more than POOL_MIN_TILES tiles (decode_params.h); how many are there follows from the
+  // position, as it does in that kernel. Set only where the merge is launched right behind the split-K kernel.
+  const int* pos0;
+  int base_pos, n_local, n_ctx;
 };
 constexpr int XBUF_HEADER_BYTES = 256;
 

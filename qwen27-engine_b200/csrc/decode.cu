@@ -135,8 +135,6 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constant__
               const DecodeParams p) {
   using G = Geo<Q8>;
   constexpr int NSTAGE = G::NSTAGE;
-  pdl_wait();
-  pdl_trigger();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sgen = smem_raw + (sbase - smem_u32(smem_raw));
@@ -151,7 +149,13 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constant__
       tma_prefetch_desc(&tm_ks);
       tma_prefetch_desc(&tm_vs);
     }
+    for (int s = 0; s < NSTAGE; s++) mbar_init(&full[s], 1);
+    *abort_flag = 0;
+    for (int i = 0; i < 2 * NGROUP; i++) ((volatile uint32_t*)(sgen + OFF_TOK))[i] = 0;
+    mbar_fence_init();
   }
+  pdl_wait();
+  pdl_trigger();  // after the wait: when the merge kernel's CTAs start, everything before this kernel has completed
   const int ch = blockIdx.x, kh = blockIdx.y;
   const int T = p.T, R = GQA * T;
   const int seq = PAGED ? blockIdx.z : 0;
@@ -174,20 +178,14 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constant__
   float* out = p.part + (((size_t)seq * p.nkvh + kh) * p.nch + ch) * MAXR * PROW;
 
   if (c0 >= c1) {
-    // Empty chunk: neutral partial (src/attn.cu:117-120). The paged merge reads only the chunks
-    // that a sequence has, so there nothing is written.
-    if (!PAGED)
+    // Empty chunk: what the merge reads of it is the neutral partial (src/attn.cu:117-120). It reads only the
+    // partials that hold something (filled_chunks; with pages the chunks that a sequence has).
+    if (!PAGED && ch < filled_chunks(n, p.nch))
       for (int i = tid; i < R * PROW; i += N_THREADS) out[i] = (i % PROW == 0) ? M_INIT : 0.f;
     return;
   }
   const int ntiles = (c1 - c0 + TILE - 1) / TILE;
 
-  if (tid == 0) {
-    for (int s = 0; s < NSTAGE; s++) mbar_init(&full[s], 1);
-    *abort_flag = 0;
-    for (int i = 0; i < 2 * NGROUP; i++) ((volatile uint32_t*)(sgen + OFF_TOK))[i] = 0;
-    mbar_fence_init();
-  }
   __syncthreads();
 
   // TMA of tile `it` into stage it % NSTAGE (one thread).
@@ -596,7 +594,7 @@ int launch_decode(const CUtensorMap* kv, const CUtensorMap* ks, const CUtensorMa
       attr[dev] = true;
     }
   }
-  Q27B_CK(launch_pdl(decode_kernel<NT, PAGED, Q8>, dim3(p.nch, p.nkvh, nseq), dim3(N_THREADS), SMEM_BYTES, s, *kv, *ks, *vv,
+  Q27B_CK(launch_step(decode_kernel<NT, PAGED, Q8>, dim3(p.nch, p.nkvh, nseq), dim3(N_THREADS), SMEM_BYTES, s, *kv, *ks, *vv,
                      *vs, p));
   return Q27B_OK;
 }
@@ -641,6 +639,11 @@ int launch_q8(const CUtensorMap* kv, const CUtensorMap* ks, const CUtensorMap* v
   if (k == 0 || k == 3) return launch_decode_ws(kv, ks, vv, vs, p, paged, nseq, s, single_group);
   if (k == 4) return launch_decode_wt(kv, ks, vv, vs, p, paged, nseq, s);
   return paged ? launch_decode_t<true, true>(kv, ks, vv, vs, p, nseq, s) : launch_decode_t<false, true>(kv, ks, vv, vs, p, nseq, s);
+}
+
+// The merge's view of how many partials the split-K kernel writes.
+void set_filled(MergeParams& mp, const int* pos0, int base_pos, int n_local, int n_ctx) {
+  mp.pos0 = pos0; mp.base_pos = base_pos; mp.n_local = n_local; mp.n_ctx = n_ctx;
 }
 
 // Records a measurement event on s; in a stream that is being captured the record becomes an event
@@ -748,6 +751,7 @@ int q27b_attn_decode(const float* qn, const float* qg, const void* kcache, const
   MergeParams mp = {};
   mp.part = ctx->dec.p; mp.nparts = nch; mp.rows = (int64_t)T * nqh; mp.qg = qg; mp.o = o; mp.xq = xq; mp.xd = xd;
   mp.T = T; mp.nqh = nqh;
+  set_filled(mp, pos0, 0, -1, n_ctx);
   return launch_merge(mp, true, (cudaStream_t)stream);
 }
 
@@ -766,6 +770,7 @@ int q27b_attn_decode_partial(const float* qn, const void* kcache, const void* vc
     return rc;
   MergeParams mp = {};
   mp.part = ctx->dec.p; mp.nparts = nch; mp.rows = (int64_t)T * nqh; mp.part_out = part; mp.T = T; mp.nqh = nqh;
+  set_filled(mp, pos0, base_pos, n_local, n_ctx);
   return launch_merge(mp, true, (cudaStream_t)stream);
 }
 
@@ -793,6 +798,7 @@ int q27b_attn_decode_partial_push(const float* qn, const void* kcache, const voi
   mp.part = ctx->dec.p; mp.nparts = nch; mp.rows = (int64_t)T * nqh; mp.T = T; mp.nqh = nqh;
   for (int k = 0; k < nz; k++) mp.push_buf[k] = peer_xbuf[k];
   mp.push_n = nz; mp.push_z = my_z; mp.xbuf = (int*)peer_xbuf[my_z]; mp.status = ctx->status;
+  set_filled(mp, pos0, base_pos, n_local, n_ctx);
   return launch_merge(mp, true, (cudaStream_t)stream);
 }
 
@@ -833,6 +839,7 @@ int q27b_attn_decode_exchange(const float* qn, const float* qg, const void* kcac
   mp.part = ctx->dec.p; mp.nparts = nch_out; mp.rows = rows; mp.T = T; mp.nqh = nqh; mp.qg = qg; mp.o = o;
   for (int k = 0; k < nz; k++) mp.push_buf[k] = peer_xbuf[k];
   mp.push_n = nz; mp.push_z = my_z; mp.xbuf = (int*)peer_xbuf[my_z]; mp.status = ctx->status;
+  set_filled(mp, pos0, base_pos, n_local, n_ctx);
   return launch_merge(mp, true, (cudaStream_t)stream);
 }
 
@@ -868,6 +875,7 @@ int q27b_attn_decode_noalloc(const float* qn, const float* qg, const void* kcach
   MergeParams mp = {};
   mp.part = g_noalloc_part_ptr[dev]; mp.nparts = nch; mp.rows = (int64_t)T * nqh; mp.qg = qg; mp.o = o; mp.xq = xq;
   mp.xd = xd; mp.T = T; mp.nqh = nqh;
+  set_filled(mp, pos0, 0, -1, n_ctx);
   return launch_merge(mp, true, (cudaStream_t)stream);
 }
 

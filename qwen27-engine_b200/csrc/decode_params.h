@@ -25,6 +25,17 @@ struct DecodeParams {
   unsigned long long* trace;
 };
 
+// One sequence: its tiles of 64 positions are dealt out to the nch chunks of a KV head in equal shares of up to
+// ceil(tiles / nch) tiles; above this share the chunks keep back a common pool (decode_ws.cu) and every chunk has tiles.
+constexpr int POOL_MIN_TILES = 8;
+// How many of the nch partials of a KV head hold anything when n positions are attended (at least one: the first
+// chunk's partial is always written).
+__host__ __device__ inline int filled_chunks(int n, int nch) {
+  const int tiles = (n + 63) / 64, share = (tiles + nch - 1) / nch;
+  if (share > POOL_MIN_TILES) return nch;
+  return tiles < 1 ? 1 : (tiles + share - 1) / share;
+}
+
 // Split-K decode over a q8_0 cache on the tcgen05 path (decode_tc.cu). Same grid, same partial
 // layout and same tensor maps as the warp-MMA kernel. paged: rows through the page table.
 int launch_decode_tc(const CUtensorMap* kv, const CUtensorMap* ks, const CUtensorMap* vv, const CUtensorMap* vs,

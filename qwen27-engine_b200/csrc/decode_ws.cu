@@ -150,8 +150,6 @@ __global__ void __launch_bounds__(256 * NG, 3 - NG)
 decode_ws_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constant__ CUtensorMap tm_ks,
                  const __grid_constant__ CUtensorMap tm_vv, const __grid_constant__ CUtensorMap tm_vs,
                  const DecodeParams p) {
-  pdl_wait();
-  pdl_trigger();
   using L = Lay<NG>;
   constexpr int WS_THREADS = L::THREADS;
   constexpr int OFF_KRING = L::OFF_KRING, OFF_VRING = L::OFF_VRING, OFF_Q = L::OFF_Q, OFF_P = L::OFF_P, OFF_MAX = L::OFF_MAX,
@@ -178,7 +176,15 @@ decode_ws_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constan
     tma_prefetch_desc(&tm_vv);
     tma_prefetch_desc(&tm_ks);
     tma_prefetch_desc(&tm_vs);
+    for (int s = 0; s < NG * (KDEPTH + VDEPTH); s++) mbar_init(&fullK[s], 1);
+    *abort_flag = 0;
+    for (int i = 0; i < 8; i++) ((volatile uint32_t*)(sgen + OFF_TOK))[i] = 0;
+    mbar_fence_init();
   }
+  // What does not touch global memory runs while the previous kernel of the stream (the prologue that writes the
+  // query and the new rows) drains.
+  pdl_wait();
+  pdl_trigger();  // after the wait: when the merge kernel's CTAs start, everything before this kernel has completed
   const int ch = blockIdx.x, kh = blockIdx.y;
   const int T = p.T, R = GQA * T;
   const int seq = PAGED ? blockIdx.z : 0;
@@ -215,7 +221,7 @@ decode_ws_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constan
   } else {
     ntiles_all = (n + TILE - 1) / TILE;
     const int share = (ntiles_all + p.nch - 1) / p.nch;
-    const int own = (p.sched && share > 8) ? share - max(2, share >> 3) - (share >> 4) : share;
+    const int own = (p.sched && share > POOL_MIN_TILES) ? share - max(2, share >> 3) - (share >> 4) : share;
     t_first = ch * own;
     n_static = max(0, min(own, ntiles_all - t_first));
     pool0 = p.nch * own;
@@ -225,19 +231,13 @@ decode_ws_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constan
   float* out = p.part + (((size_t)seq * p.nkvh + kh) * p.nch + ch) * MAXR * PROW;
 
   if (n_static == 0 && !has_pool) {
-    // Nothing to do: neutral partial (src/attn.cu:117-120). The paged merge reads only the chunks
-    // that a sequence has, so there nothing is written.
-    if (!PAGED)
+    // Nothing to do. The merge reads only the partials that hold something (filled_chunks; with pages the chunks
+    // that a sequence has): anything else it reads is the neutral partial (src/attn.cu:117-120).
+    if (!PAGED && ch < filled_chunks(n, p.nch))
       for (int i = tid; i < R * PROW; i += WS_THREADS) out[i] = (i % PROW == 0) ? M_INIT : 0.f;
     return;
   }
 
-  if (tid == 0) {
-    for (int s = 0; s < NG * (KDEPTH + VDEPTH); s++) mbar_init(&fullK[s], 1);
-    *abort_flag = 0;
-    for (int i = 0; i < 8; i++) ((volatile uint32_t*)(sgen + OFF_TOK))[i] = 0;
-    mbar_fence_init();
-  }
   __syncthreads();
   if (tid == 0) stamp(1);
 
@@ -786,9 +786,9 @@ int launch_ws_nt(const CUtensorMap* kv, const CUtensorMap* ks, const CUtensorMap
                  const DecodeParams& p, bool paged, int nseq, cudaStream_t s) {
   const dim3 grid(p.nch, p.nkvh, nseq);
   if (paged)
-    Q27B_CK(launch_pdl(decode_ws_kernel<NT, true, NG>, grid, dim3(Lay<NG>::THREADS), Lay<NG>::SMEM_BYTES, s, *kv, *ks, *vv, *vs, p));
+    Q27B_CK(launch_step(decode_ws_kernel<NT, true, NG>, grid, dim3(Lay<NG>::THREADS), Lay<NG>::SMEM_BYTES, s, *kv, *ks, *vv, *vs, p));
   else
-    Q27B_CK(launch_pdl(decode_ws_kernel<NT, false, NG>, grid, dim3(Lay<NG>::THREADS), Lay<NG>::SMEM_BYTES, s, *kv, *ks, *vv, *vs, p));
+    Q27B_CK(launch_step(decode_ws_kernel<NT, false, NG>, grid, dim3(Lay<NG>::THREADS), Lay<NG>::SMEM_BYTES, s, *kv, *ks, *vv, *vs, p));
   return Q27B_OK;
 }
 

@@ -249,7 +249,7 @@ decode_wt_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constan
   } else {
     ntiles_all = (n + TILE - 1) / TILE;
     const int share = (ntiles_all + p.nch - 1) / p.nch;
-    const int own = (p.sched && share > 8) ? share - max(2, share >> 3) - (share >> 4) : share;
+    const int own = (p.sched && share > POOL_MIN_TILES) ? share - max(2, share >> 3) - (share >> 4) : share;
     t_first = ch * own;
     n_static = max(0, min(own, ntiles_all - t_first));
     pool0 = p.nch * own;

@@ -22,12 +22,12 @@ using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, voi
 EncodeFn g_encode = nullptr;
 }  // namespace
 
-bool pdl_enabled() {
-  static const bool on = [] {
+PdlMode pdl_mode() {
+  static const PdlMode m = [] {
     const char* e = getenv("Q27_PDL");
-    return e && e[0] == '1';
+    return !e ? PDL_STEP : e[0] == '1' ? PDL_ALL : PDL_NONE;
   }();
-  return on;
+  return m;
 }
 
 int fail(int code, const std::string& msg) {

@@ -65,15 +65,17 @@ int paged_ws(DeviceCtx* ctx, size_t floats, float** out);
 // instead when not even two pieces fit.
 int fit_prefill_split(DeviceCtx* ctx, int* ts, int* ns, int tokens, int nqh, bool must_merge, float** part);
 
-// True when Q27_PDL=1, the reference's switch with the reference's default (off; src/ops.cu:12-15,
-// src/common.cuh:28-42): kernels are then launched with the programmatic-stream-serialization
-// attribute, so a kernel's CTAs may be scheduled while its predecessor drains (every kernel here
-// begins with griddepcontrol.wait, which holds it until the predecessor has completed and flushed).
-// Measured on B200 it does not pay for this pair of kernels (the 226 KB CTAs cannot co-reside).
-bool pdl_enabled();
+// The switch Q27_PDL of the reference (src/ops.cu:12-15, src/common.cuh:28-42): a kernel launched with the
+// programmatic-stream-serialization attribute may be scheduled while its predecessor drains; griddepcontrol.wait
+// in the kernel holds it until the predecessor has completed and flushed. Q27_PDL=1: every kernel, 0: none,
+// unset: the kernels of a decode step (launch_step), which do what needs no memory - barriers, tensor-map
+// prefetch, index arithmetic - before they wait. PDL_ALL / PDL_STEP / PDL_NONE.
+enum PdlMode { PDL_NONE = 0, PDL_STEP = 1, PDL_ALL = 2 };
+PdlMode pdl_mode();
 
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
+inline cudaError_t launch_attr(bool overlap, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                               Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -81,10 +83,19 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+  attr[0].val.programmaticStreamSerializationAllowed = overlap ? 1 : 0;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
+  return launch_attr(pdl_mode() == PDL_ALL, kern, grid, block, smem, s, static_cast<Args&&>(args)...);
+}
+// Kernels of a decode step.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_step(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
+  return launch_attr(pdl_mode() != PDL_NONE, kern, grid, block, smem, s, static_cast<Args&&>(args)...);
 }
 
 // The same through a process-wide cache keyed by every argument and the current device (caches of the

@@ -85,7 +85,6 @@ __device__ __forceinline__ void store_row(const float (&a)[4], const float (&b)[
 // Grid: ceil(jobs / 8) CTAs of 8 warps; job = (token, row kind). With norm: nqh query rows, then
 // nkvh K rows, then nkvh V rows per token; without: K rows then V rows.
 __global__ void __launch_bounds__(256) prep_kernel(const PrepParams p) {
-  pdl_wait();
   pdl_trigger();
   const int lane = threadIdx.x & 31;
   const bool norm = p.q_norm != nullptr;
@@ -96,15 +95,26 @@ __global__ void __launch_bounds__(256) prep_kernel(const PrepParams p) {
   const int tok = job / per_tok;  // with pages: sequence * T + token
   int r = job % per_tok;
   const int seq = paged ? tok / p.T : 0;
-  const int pos = paged ? p.seq_len[seq] - p.T + tok % p.T : *p.pos0 + tok;
-  if (pos < 0 || pos >= p.n_ctx) return;  // never write outside the cache
   const bool isq = norm && r < p.nqh;
   if (norm && !isq) r -= p.nqh;
   const bool isv = !isq && r >= p.nkvh;
   const int head = isq ? r : (isv ? r - p.nkvh : r);
   const float* src = isq ? p.qg + ((size_t)tok * p.nqh + head) * 512
                          : (isv ? p.v : p.k) + ((size_t)tok * p.nkvh + head) * AD;
+  // Everything above is index arithmetic and runs while the previous kernel drains. All loads are requested
+  // before the first one is used: the position (and with pages the page index behind it) is one chain of
+  // round trips, the row and the norm weights another.
+  pdl_wait();
+  const int pos = paged ? p.seq_len[seq] - p.T + tok % p.T : *p.pos0 + tok;
   const float4 fa = *(const float4*)(src + 4 * lane), fb = *(const float4*)(src + 128 + 4 * lane);
+  const float* w = isq ? p.q_norm : p.k_norm;
+  float4 wa = {}, wb = {};
+  if (norm && !isv) {
+    wa = *(const float4*)(w + 4 * lane);
+    wb = *(const float4*)(w + 128 + 4 * lane);
+  }
+  if (pos < 0 || pos >= p.n_ctx) return;  // never write outside the cache
+  const int pg = paged && !isq ? p.page_table[(size_t)seq * p.max_pages + pos / Q27B_PAGE] : 0;
   float a[4] = {fa.x, fa.y, fa.z, fa.w}, b[4] = {fb.x, fb.y, fb.z, fb.w};
 
   if (norm && !isv) {
@@ -114,8 +124,6 @@ __global__ void __launch_bounds__(256) prep_kernel(const PrepParams p) {
     for (int i = 0; i < 4; i++) t += a[i] * a[i] + b[i] * b[i];
     t = warp_sum(t);
     const float scale = rsqrtf(t / 256 + p.eps);
-    const float* w = isq ? p.q_norm : p.k_norm;
-    const float4 wa = *(const float4*)(w + 4 * lane), wb = *(const float4*)(w + 128 + 4 * lane);
     const float wav[4] = {wa.x, wa.y, wa.z, wa.w}, wbv[4] = {wb.x, wb.y, wb.z, wb.w};
 #pragma unroll
     for (int i = 0; i < 4; i++) {
@@ -150,7 +158,6 @@ __global__ void __launch_bounds__(256) prep_kernel(const PrepParams p) {
     store_row(a, b, isv ? p.vcache : p.kcache, (size_t)head * p.n_ctx + pos, lane, (size_t)p.nkvh * p.n_ctx, p.q8 != 0);
     return;
   }
-  const int pg = p.page_table[(size_t)seq * p.max_pages + pos / Q27B_PAGE];
   if (pg < 0 || pg >= p.n_pages) {  // never write outside the pool: flag it and drop the row
     if (lane == 0) atomicOr(p.status, ST_BAD_PAGE);
     return;
@@ -162,8 +169,7 @@ __global__ void __launch_bounds__(256) prep_kernel(const PrepParams p) {
 int launch_prep(const PrepParams& p, cudaStream_t s) {
   const int per_tok = (p.q_norm ? p.nqh : 0) + 2 * p.nkvh;
   const int jobs = (p.page_table ? p.B : 1) * p.T * per_tok;
-  prep_kernel<<<(jobs + 7) / 8, 256, 0, s>>>(p);
-  Q27B_CK(cudaGetLastError());
+  Q27B_CK(launch_step(prep_kernel, dim3((jobs + 7) / 8), dim3(256), 0, s, p));
   return Q27B_OK;
 }
 

@@ -305,3 +305,63 @@ def test_peer_memory_merge_reports_a_missing_slice(q27):
     assert q27.device_status() == 0
     assert torch.equal(o, want)
     assert int(buf[:4].view(torch.int32).item()) == 1  # the step counter advanced from zero
+
+
+@pytest.mark.parametrize("n", [1, 64, 65, 2368, 2369, 18944, 18945])
+def test_empty_chunks_leave_no_trace(q27, orc, n):
+    """Chunks without a tile write no partial (37 chunks of a KV head: 64 positions fill one, 2,368 all of them; from
+    18,945 on there is a tile pool): whatever an earlier call left in the workspace must not be merged."""
+    T, nkvh = 1, 4
+    nqh = nkvh * GQA
+    nan = torch.full((T, nqh, AD), float("nan"), device="cuda")
+    kc = q27.new_cache(nkvh, 20000)
+    q27.attn_decode(nan, torch.zeros((T, nqh, 512), device="cuda"), kc, kc, torch.empty_like(nan), None, None,
+                    pos_tensor(20000 - T), T, SCALE, nqh, nkvh, 20000)
+    run_decode(q27, orc, T, nkvh, n)
+    assert q27.device_status() == 0
+
+
+def test_step_captured_behind_a_copy_and_another_stream(q27, orc):
+    """The kernels of a step start while their predecessor drains; in a graph the predecessor may also be a copy or a
+    join of two streams. The position changes between replays."""
+    from qwen27_engine_b200 import synth
+    T, nkvh, n_ctx = 2, 2, 4000
+    nqh = nkvh * GQA
+    eps, theta = 1e-6, 10000000.0 ** (-2.0 / 64)
+    _, _, kf, vf = synth.decode_inputs(T, nqh, nkvh, n_ctx)
+    kc_ref, vc_ref = orc.fill_cache(kf, vf, n_ctx)
+    rn = lambda seed, *s: dev(synth.normal(seed, s))  # noqa: E731
+    qg, k, v = rn(synth.SEED_Q, T, nqh, 512), rn(synth.SEED_K, T, nkvh, AD), rn(synth.SEED_V, T, nkvh, AD)
+    w = torch.ones(AD, device="cuda")
+    pos_in, pos, qg_in = pos_tensor(0), pos_tensor(0), qg.clone()
+    kc, vc = dev(kc_ref), dev(vc_ref)
+    qn, o = torch.empty((T, nqh, AD), device="cuda"), torch.empty((T, nqh, AD), device="cuda")
+
+    def step(qn, o, kc, vc):
+        q27.attn_prep(qg, k, v, w, w, qn, kc, vc, pos, T, eps, theta, nqh, nkvh, n_ctx)
+        q27.attn_decode(qn, qg, kc, vc, o, None, None, pos, T, SCALE, nqh, nkvh, n_ctx)
+
+    side = torch.cuda.Stream()
+    step(qn, o, kc, vc)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            qg.copy_(qg_in)
+        pos.copy_(pos_in)
+        torch.cuda.current_stream().wait_stream(side)
+        step(qn, o, kc, vc)
+    for n in (100, 3000, 64):
+        kc.copy_(dev(kc_ref)), vc.copy_(dev(vc_ref))
+        pos_in.fill_(n - T)
+        g.replay()
+        torch.cuda.synchronize()
+        got = o.clone()
+        kc2, vc2 = dev(kc_ref), dev(vc_ref)
+        o2 = torch.empty_like(o)
+        step(torch.empty_like(qn), o2, kc2, vc2)
+        torch.cuda.synchronize()
+        assert_close(got.cpu().numpy(), o2.cpu().numpy(), "replay at n=%d" % n)
+        assert torch.equal(kc, kc2) and torch.equal(vc, vc2)
+    assert q27.device_status() == 0
