@@ -5,9 +5,12 @@ layer (namespace q27, src/ops.h:50-77: kv_cache_bytes, attn_prep, attn_decode, a
 attn_chunks), so that a test written against the reference reads the same here. Arguments are
 torch CUDA tensors (torch is used for device memory and streams only); every call forwards the
 raw device pointers to libq27b_attn.so and raises RuntimeError where the reference throws
-std::runtime_error. There is no CPU path: if the library cannot be loaded the import fails.
+std::runtime_error. There is no CPU path: if the library cannot be loaded the import fails. The calls
+that an engine makes per layer go through a native binding of the same checks (csrc/binding.cpp).
 """
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 
 import torch
@@ -91,6 +94,23 @@ def _stream():
 
 def _f(x):
     return ctypes.c_float(x)
+
+
+def _load_binding():
+    """The native binding of the per-layer entry points (csrc/binding.cpp), on this module's library."""
+    path = os.path.join(_HERE, "q27b_binding.so")
+    if not os.path.exists(path):
+        raise ImportError("q27b_binding.so is not built (run `python qwen27-engine_b200/build.py`); there is no fallback path")
+    loader = importlib.machinery.ExtensionFileLoader("q27b_binding", path)
+    mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("q27b_binding", loader))
+    loader.exec_module(mod)
+    fns = tuple(ctypes.cast(getattr(_lib, "q27b_" + n), ctypes.c_void_p).value
+                for n in ("attn_prep", "attn_decode", "attn_prep_paged", "attn_decode_paged", "attn_prefill"))
+    mod.bind(fns, _ptr, _check, torch.float32, torch.int32, torch.int8)
+    return mod
+
+
+_native = _load_binding()
 
 
 def kv_cache_bytes(nkvh, n_ctx, q8=True):
@@ -357,19 +377,13 @@ def kv_append(k, v, kcache, vcache, pos0, T, nkvh, n_ctx, q8=True):
 def attn_prep(qg, k, v, q_norm, k_norm, qn, kcache, vcache, pos0, T, eps, theta_scale, nqh, nkvh, n_ctx, q8=True,
               rope3=None, rdelta=None):
     """q27::attn_prep (src/ops.h:59-62)."""
-    _check(_lib.q27b_attn_prep(_ptr(qg, torch.float32), _ptr(k, torch.float32), _ptr(v, torch.float32),
-                               _ptr(q_norm, torch.float32), _ptr(k_norm, torch.float32), _ptr(qn, torch.float32),
-                               _ptr(kcache), _ptr(vcache), _ptr(pos0, torch.int32), int(T), _f(eps), _f(theta_scale),
-                               int(nqh), int(nkvh), int(n_ctx), int(bool(q8)), _stream(),
-                               _ptr(rope3, torch.int32, True), _ptr(rdelta, torch.int32, True)))
+    _native.attn_prep(qg, k, v, q_norm, k_norm, qn, kcache, vcache, pos0, T, eps, theta_scale, nqh, nkvh, n_ctx, q8,
+                      rope3, rdelta)
 
 
 def attn_decode(qn, qg, kcache, vcache, o, xq, xd, pos0, T, kq_scale, nqh, nkvh, n_ctx, q8=True):
     """q27::attn_decode (src/ops.h:66-67). With xq given the result goes to q8_1 (xq, xd) instead of o."""
-    _check(_lib.q27b_attn_decode(_ptr(qn, torch.float32), _ptr(qg, torch.float32), _ptr(kcache), _ptr(vcache),
-                                 _ptr(o, torch.float32, True), _ptr(xq, torch.int8, True),
-                                 _ptr(xd, torch.float32, True), _ptr(pos0, torch.int32), int(T), _f(kq_scale),
-                                 int(nqh), int(nkvh), int(n_ctx), int(bool(q8)), _stream()))
+    _native.attn_decode(qn, qg, kcache, vcache, o, xq, xd, pos0, T, kq_scale, nqh, nkvh, n_ctx, q8)
 
 
 def attn_decode_noalloc(qn, qg, kcache, vcache, o, xq, xd, pos0, T, kq_scale, nqh, nkvh, n_ctx, q8=True):
@@ -402,21 +416,15 @@ def lse_merge(part, nparts, part_stride, rows, qg, o, xq=None, xd=None):
 def attn_decode_paged(qn, qg, kpool, vpool, page_table, seq_len, o, B, T, kq_scale, nqh, nkvh, n_pages, max_pages,
                       max_seq_len):
     """Batched decode over a paged q8_0 cache (256-position pages)."""
-    _check(_lib.q27b_attn_decode_paged(_ptr(qn, torch.float32), _ptr(qg, torch.float32), _ptr(kpool), _ptr(vpool),
-                                       _ptr(page_table, torch.int32), _ptr(seq_len, torch.int32),
-                                       _ptr(o, torch.float32), int(B), int(T), _f(kq_scale), int(nqh), int(nkvh),
-                                       int(n_pages), int(max_pages), int(max_seq_len), _stream()))
+    _native.attn_decode_paged(qn, qg, kpool, vpool, page_table, seq_len, o, B, T, kq_scale, nqh, nkvh, n_pages, max_pages,
+                              max_seq_len)
 
 
 def attn_prep_paged(qg, k, v, q_norm, k_norm, qn, kpool, vpool, page_table, seq_len, B, T, eps, theta_scale, nqh, nkvh,
                     n_pages, max_pages, rope3=None, rdelta=None):
     """q27::attn_prep for B sequences over the page pool; with q_norm None it only appends K and V."""
-    _check(_lib.q27b_attn_prep_paged(_ptr(qg, torch.float32, True), _ptr(k, torch.float32), _ptr(v, torch.float32),
-                                     _ptr(q_norm, torch.float32, True), _ptr(k_norm, torch.float32, True),
-                                     _ptr(qn, torch.float32, True), _ptr(kpool), _ptr(vpool),
-                                     _ptr(page_table, torch.int32), _ptr(seq_len, torch.int32), int(B), int(T),
-                                     _f(eps), _f(theta_scale), int(nqh), int(nkvh), int(n_pages), int(max_pages),
-                                     _stream(), _ptr(rope3, torch.int32, True), _ptr(rdelta, torch.int32, True)))
+    _native.attn_prep_paged(qg, k, v, q_norm, k_norm, qn, kpool, vpool, page_table, seq_len, B, T, eps, theta_scale, nqh,
+                            nkvh, n_pages, max_pages, rope3, rdelta)
 
 
 def kv_page_copy(pool, src_page, dst_page, rows, nkvh, n_pages):
@@ -483,9 +491,7 @@ class Pager:
 
 def attn_prefill(qn, qg, kcache, vcache, o, pos0, M, kq_scale, nqh, nkvh, n_ctx, q8=True, depth_hint=-1):
     """q27::attn_prefill (src/ops.h:71-72)."""
-    _check(_lib.q27b_attn_prefill(_ptr(qn, torch.float32), _ptr(qg, torch.float32), _ptr(kcache), _ptr(vcache),
-                                  _ptr(o, torch.float32), _ptr(pos0, torch.int32), int(M), _f(kq_scale), int(nqh),
-                                  int(nkvh), int(n_ctx), int(bool(q8)), _stream(), int(depth_hint)))
+    _native.attn_prefill(qn, qg, kcache, vcache, o, pos0, M, kq_scale, nqh, nkvh, n_ctx, q8, depth_hint)
 
 
 def attn_prefill_q8_1(qn, qg, kcache, vcache, xq, xd, pos0, M, kq_scale, nqh, nkvh, n_ctx, q8=True, depth_hint=-1):

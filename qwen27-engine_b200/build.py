@@ -1,4 +1,5 @@
-"""Builds libq27b_attn.so (CUDA kernels + C ABI) for sm_100a, in-tree.
+"""Builds libq27b_attn.so (CUDA kernels + C ABI) for sm_100a and q27b_binding.so (the CPython binding
+of the per-layer entry points), in-tree.
 
 nvcc cross-compiles without a GPU. No fast-math flag is used anywhere: the quantisers are
 specified in IEEE operations, and the attention kernels ask for the approximate instructions
@@ -7,6 +8,7 @@ specified in IEEE operations, and the attention kernels ask for the approximate 
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -14,6 +16,7 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libq27b_attn.so")
 SOURCES = ["host.cu", "kv_append.cu", "kv_wire.cu", "combine.cu", "decode.cu", "decode_tc.cu", "decode_ws.cu", "decode_wt.cu", "decode_ref.cu", "prefill.cu", "prefill_f16.cu", "sum_norm.cu", "peak_mma.cu", "pager.cu"]
+BINDING = os.path.join(HERE, "q27b_binding.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
          "--expt-relaxed-constexpr"]
@@ -44,14 +47,35 @@ def _compile(src, verbose):
     return obj, r.stderr
 
 
+def _build_binding():
+    src = os.path.join(CSRC, "binding.cpp")
+    if not _stale(BINDING, [src]):
+        return
+    import torch
+    root = os.path.dirname(torch.__file__)
+    lib = os.path.join(root, "lib")
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           sysconfig.get_paths()["include"], "/usr/local/cuda/include"]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC",
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI]
+    for d in inc:
+        cmd += ["-isystem", d]
+    r = subprocess.run(cmd + [src, "-o", BINDING, "-L" + lib, "-Wl,-rpath," + lib, "-lc10", "-lc10_cuda", "-ltorch_cpu",
+                              "-ltorch_python"], capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("binding.cpp failed:\n%s\n%s" % (r.stdout, r.stderr))
+
+
 def build(verbose=False, force=False):
     os.makedirs(OBJ, exist_ok=True)
     if force:
         for f in os.listdir(OBJ):
             os.remove(os.path.join(OBJ, f))
     srcs = [s for s in SOURCES if os.path.exists(os.path.join(CSRC, s))]
-    with ThreadPoolExecutor(max_workers=len(srcs)) as ex:
+    with ThreadPoolExecutor(max_workers=len(srcs) + 1) as ex:
+        binding = ex.submit(_build_binding)
         res = list(ex.map(lambda s: _compile(s, verbose), srcs))
+        binding.result()
     objs = [o for o, _ in res]
     if verbose:
         for _, log in res:

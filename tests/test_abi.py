@@ -5,6 +5,7 @@ import os
 import re
 
 import pytest
+import torch
 
 from conftest import ROOT
 
@@ -236,3 +237,30 @@ def test_sum_push_refuses_a_null_buffer_before_any_cuda_call(q27):
     bufs = (ctypes.c_void_p * 2)(ctypes.c_void_p(16), ctypes.c_void_p(0))
     assert lib.q27b_sum_push(ctypes.c_void_p(16), 5120, 4, 0, 2, bufs, ctypes.c_void_p(0)) == q27.BAD_SHAPE
     assert b"null exchange buffer" in lib.q27b_last_error()
+
+
+def test_native_binding_checks_like_the_python_layer(q27):
+    """The natively bound entry points raise what the ctypes layer raises, argument by argument (no CUDA call is
+    reached): dtype and device of tensors, null tensors, raw addresses, number conversions, keywords."""
+    t, sub = torch.zeros(4), torch.nn.Parameter(torch.zeros(4))
+    args = [0] * 5 + [None, None, 0, 4, 0.1, 24, 4, 100]
+    for bad in (t, sub, t[::2]):
+        for i in (0, 2, 7):
+            a = list(args)
+            a[i] = bad
+            with pytest.raises(q27.Q27Error, match="contiguous CUDA tensors") as e:
+                q27.attn_decode(*a)
+            assert e.value.code == q27.BAD_SHAPE
+    a = list(args)
+    a[1] = None
+    with pytest.raises(q27.Q27Error, match="null tensor"):
+        q27.attn_decode(*a)
+    for i, bad, kind in ((8, "x", ValueError), (8, None, TypeError), (9, "x", TypeError), (10, [], TypeError)):
+        a = list(args)
+        a[i] = bad
+        with pytest.raises(kind):
+            q27.attn_decode(*a)
+    with pytest.raises(TypeError):
+        q27.attn_decode(*args[:-1])
+    with pytest.raises(AttributeError):
+        q27.attn_prefill("not a tensor", *args[1:5], 0, 4, 0.1, 24, 4, 100)
