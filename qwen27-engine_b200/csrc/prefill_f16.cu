@@ -249,25 +249,47 @@ prefill_f16_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     const int wg = warp >> 2, q = warp & 3;
     const int r = q * 32 + lane;       // query row = TMEM lane
     const int t = (row0 + r) / GQA, h = kh * GQA + (row0 + r) % GQA;
-    const bool live = t < p.M;
     float* xch = (float*)(sgen + OFF_XCH);
     const uint32_t tlane = tmem + ((uint32_t)(q * 32) << 16);
     {
       // Q tile -> tensor memory, the A operand of every Q K^T MMA of this CTA (lane = row, column c =
       // dims 2c, 2c+1 as f16, even dim in the low half): it is read from there 16 times per tile
-      // without touching shared memory. This thread writes dims OW wg .. OW wg + OW - 1 of its row,
-      // scaled and rounded to f16; rows past M are zero.
-      const float* src = live ? p.qn + ((size_t)t * p.nqh + h) * AD + OW * wg : nullptr;
+      // without touching shared memory. This warp writes dims OW wg .. OW wg + OW - 1 of its 32 rows,
+      // scaled and rounded to f16; rows past M are zero. 32 dims at a time, loaded with eight lanes to 128
+      // contiguous bytes of a row and turned to a row per thread in the P buffer (64 bytes a row, 16-byte chunk c of
+      // row r at c ^ (r / 2 % 4)). With the epilogue below: 50 tokens behind 3,000 on an f16 cache 46.6 -> 36.7 us.
+      uint8_t* stage = sgen + OFF_P + (warp & 7) * 2048;  // room for eight warps: with four warpgroups they take turns
+      static_assert(8 * 2048 <= P_BYTES, "staging of the Q tile");
 #pragma unroll 1
-      for (int c = 0; c < OW / 64; c++) {
-        uint32_t w[32];
+      for (int turn = 0, c = 0; turn < (NWG + 1) / 2; turn++, c = 0) {
+        if (turn > 0) row_sync<NWG>(q);
+        if ((wg >> 1) != turn) continue;
+#pragma unroll 1
+        for (; c < OW / 32; c++) {
+          float4 x[8];
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const float4 a = src ? *(const float4*)(src + c * 64 + 2 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
-          w[i] = pack_h2(a.x * p.kq_scale, a.y * p.kq_scale);
-          w[i + 1] = pack_h2(a.z * p.kq_scale, a.w * p.kq_scale);
+          for (int i = 0; i < 8; i++) {
+            const int gr = row0 + q * 32 + 4 * i + (lane >> 3), tt = gr / GQA;
+            x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (tt < p.M)
+              x[i] = *(const float4*)(p.qn + ((size_t)tt * p.nqh + kh * GQA + gr % GQA) * AD + OW * wg + c * 32 + 4 * (lane & 7));
+          }
+#pragma unroll
+          for (int i = 0; i < 8; i++) {
+            const int rr = 4 * i + (lane >> 3), ch = ((lane & 7) >> 1) ^ ((rr >> 1) & 3);
+            *(uint2*)(stage + rr * 64 + ch * 16 + (lane & 1) * 8) =
+                make_uint2(pack_h2(x[i].x * p.kq_scale, x[i].y * p.kq_scale), pack_h2(x[i].z * p.kq_scale, x[i].w * p.kq_scale));
+          }
+          __syncwarp();
+          uint32_t w[16];
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            const uint4 u = *(const uint4*)(stage + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4));
+            w[4 * i] = u.x; w[4 * i + 1] = u.y; w[4 * i + 2] = u.z; w[4 * i + 3] = u.w;
+          }
+          tmem_st16(tlane + TM_Q + wg * (OW / 2) + c * 16, w);
+          __syncwarp();
         }
-        tmem_st32(tlane + TM_Q + wg * (OW / 2) + c * 32, w);
       }
       tc_wait_st();
       tc_fence_before();
@@ -388,36 +410,47 @@ prefill_f16_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     mbar_wait(&bar[B_ODONE], 0, abort_flag, p.status);
     tc_fence_after();
     const float inv_l = 1.0f / l;
-    float* po = nsplit > 1 ? p.part + (((size_t)z * p.Ms + t) * p.nqh + h) * PROW : nullptr;
-    if (live && po && wg == 0) {
-      po[0] = m_ref;
-      po[1] = l;
-    }
+    if (nsplit > 1 && wg == 0 && t < p.M)
+      *(float2*)(p.part + (((size_t)z * p.Ms + t) * p.nqh + h) * PROW) = make_float2(m_ref, l);
+    // 32 columns at a time through shared memory (the K buffers are free now): TMEM gives a thread a row, and a row per
+    // thread would touch 32 lines with every load of the gate and every store; read back, eight lanes share 128
+    // contiguous bytes of a row.
+    uint8_t* stage = sgen + OFF_K + warp * 4096;
 #pragma unroll 1
     for (int c = 0; c < OW / 32; c++) {
       const int d0 = wg * OW + c * 32;
-      uint32_t v[32];
-      tmem_ld32(tlane + TM_O + d0, v);
-      tc_wait_ld();
-      if (!live) continue;
-      if (po) {
+      {
+        uint32_t v[32];
+        tmem_ld32(tlane + TM_O + d0, v);
+        tc_wait_ld();
+        const float f = nsplit > 1 ? 1.f : inv_l;
 #pragma unroll
-        for (int i = 0; i < 32; i += 2)
-          *(float2*)(po + 2 + d0 + i) = make_float2(__uint_as_float(v[i]), __uint_as_float(v[i + 1]));
-      } else {
-        const float* gt = p.qg + ((size_t)t * p.nqh + h) * 512 + 256 + d0;
-        float* dst = p.o + ((size_t)t * p.nqh + h) * AD + d0;
-#pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-          const float4 gg = *(const float4*)(gt + i);
-          float4 y;
-          y.x = (__uint_as_float(v[i]) * inv_l) * (1.0f / (1.0f + __expf(-gg.x)));
-          y.y = (__uint_as_float(v[i + 1]) * inv_l) * (1.0f / (1.0f + __expf(-gg.y)));
-          y.z = (__uint_as_float(v[i + 2]) * inv_l) * (1.0f / (1.0f + __expf(-gg.z)));
-          y.w = (__uint_as_float(v[i + 3]) * inv_l) * (1.0f / (1.0f + __expf(-gg.w)));
-          *(float4*)(dst + i) = y;
+        for (int i = 0; i < 8; i++)
+          *(float4*)(stage + swz128(lane, i)) = make_float4(__uint_as_float(v[4 * i]) * f, __uint_as_float(v[4 * i + 1]) * f,
+                                                            __uint_as_float(v[4 * i + 2]) * f, __uint_as_float(v[4 * i + 3]) * f);
+      }
+      __syncwarp();
+#pragma unroll 4
+      for (int i = 0; i < 8; i++) {
+        const int rr = 4 * i + (lane >> 3), gr = row0 + q * 32 + rr, tt = gr / GQA;
+        if (tt >= p.M) continue;
+        const size_t th = (size_t)tt * p.nqh + kh * GQA + gr % GQA;
+        const int d = d0 + 4 * (lane & 7);
+        float4 y = *(const float4*)(stage + swz128(rr, lane & 7));
+        if (nsplit > 1) {
+          float* po = p.part + ((size_t)z * p.Ms * p.nqh + th) * PROW + 2 + d;
+          *(float2*)po = make_float2(y.x, y.y);
+          *(float2*)(po + 2) = make_float2(y.z, y.w);
+        } else {
+          const float4 gg = *(const float4*)(p.qg + th * 512 + 256 + d);
+          y.x *= 1.0f / (1.0f + __expf(-gg.x));
+          y.y *= 1.0f / (1.0f + __expf(-gg.y));
+          y.z *= 1.0f / (1.0f + __expf(-gg.z));
+          y.w *= 1.0f / (1.0f + __expf(-gg.w));
+          *(float4*)(p.o + th * AD + d) = y;
         }
       }
+      __syncwarp();
     }
     tc_fence_before();
   } else if (warp == TMA_WARP) {
