@@ -13,20 +13,40 @@
 // tiles. The rows of a KV head are its M * 6 (token, head) pairs, token-major: a tile spans 22 tokens of all
 // six heads, so that only the last tile of a KV head has empty rows (tiles of 128 tokens of one head: 16 tokens
 // behind 30,000 took 293 us, now 64; 131 behind 30,011 521, now 274) and fewer position tiles are half masked.
-// Roles (14 warps):
+// Roles (16 warps):
 //   warps 0-7   softmax, two warpgroups: both own the 128 rows (warp w and w+4 share TMEM lanes
 //               32(w%4)..), warpgroup 0 takes positions 0-31 of a tile, warpgroup 1 positions
-//               32-63. Each thread reads its half of the per-block int32 accumulators from TMEM,
-//               applies the block scales with packed f32x2 arithmetic, exchanges the row maximum
-//               with its partner thread, writes its half of P (f16) into shared memory in the
-//               tensor core's K-major 128B-swizzled layout, rescales its half of O when the
-//               reference max moves, and writes its half of the output columns.
-//   warps 8-11  converter: V tile int8 -> f16 into the MN-major 128B-swizzled layout that the P V
-//               MMA reads directly (no transpose), and the K scales f16 -> f32 table.
+//               32-63. They read the per-block int32 accumulators from TMEM, apply the block scales with
+//               packed f32x2 arithmetic, agree with their partner warp on whether a reference max moves,
+//               write P (f16) into shared memory in the tensor core's K-major 128B-swizzled layout,
+//               rescale half of O when a reference max moves, and write half of the output columns.
+//   warps 8-11  converter: the K scales f16 -> f32 table, then the V tile int8 -> f16 into the MN-major
+//               128B-swizzled layout that the P V MMA reads directly (no transpose).
 //   warp 12     TMA producer (one lane): K and V tiles, double buffered.
 //   warp 13     MMA issuer (one lane): per tile 8 x (128x64x32 int8) into a 4-slot ring of TMEM
-//               accumulators, then 4 x (128x256x16 f16) into the O accumulator; owns TMEM.
+//               accumulators (two pairs), then 4 x (128x256x16 f16) into the O accumulator; owns TMEM.
+//   warps 14-15 idle: they complete the warpgroup whose registers setmaxnreg hands to the softmax warps
+//               (176 a thread there, 96 converter, 64 the rest; with 128 for everybody the loop spilled).
 // TMEM: columns 0-255 O (f32), 256-511 four S slots of 64 columns (s32).
+//
+// What bounds it: the SIMT lanes of the softmax warps, two warps on each quarter of the SM, which share rows and so
+// run through the same phases together. Per tile (clock stamps, 148,000 positions): 4,300 cycles at first, of them
+// 2,500 in the scale loop, 680 for the row maxima, 740 for exp and P, 450 waiting for barriers that had long
+// completed. What was changed (2,048 tokens behind 148,000, 13.7 ms before, 11.8 now):
+//  * The accumulators are read in the fragment layout of a warp MMA (tcgen05.ld.16x256b): a thread holds 4 rows x 8
+//    positions instead of 1 x 32, and loads 8 K scales and 4 Q scales per block instead of 32 and 1. A 16-byte
+//    shared-memory load returns 512 bytes to the warp whether its threads read one address or 32.
+//  * No int -> float conversion: an MMA of constants (-128 * -128 * 32 = 2^19, for two slots at once) puts an offset
+//    under the block sums, so that they are positive and below 2^20; read as bits of a float, such an integer n is the
+//    subnormal n * 2^-149, and one FMA with the K scale (times 2^110) takes the offset off again and rounds once:
+//    dk * I as exactly as the converted form. The powers of two cancel against the Q scale (times 2^39).
+//  * A vote of the two warps of a row quarter (bar.red) replaces the exchange of row maxima; maxima are exchanged only
+//    when one moves.
+//  * The scale table has a barrier of its own and is ready long before V; the softmax warps wait for neither: the
+//    issuer does before the tile's first MMA, and its commits cover the P V of two tiles back, which frees the P buffer.
+// Measured and taken back: four tcgen05.ld before one wait (64 registers; 7 % slower: the two warps of a quarter then
+// load and compute in step), the next half requested while one is scaled (2 %), four softmax warpgroups (12 %), the
+// query loads of the prologue shared by eight lanes to a row (10 % on a chunk without a prefix: eight times the divisions).
 #include "combine.h"
 #include "common.cuh"
 #include "prefill_f16.h"
@@ -37,6 +57,19 @@
 namespace q27b {
 namespace {
 
+// Bounded wait, short enough to be inlined everywhere: setmaxnreg and calls do not go together (ptxas then gives the
+// register split up), so mbar_wait, whose polling loop is a function, cannot be used. A poll may suspend the thread for
+// WAIT_HINT_NS, so that the limit is some seconds; a stuck CTA drains as described there.
+__device__ __forceinline__ void pf_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
+  if (mbar_try_wait(bar, parity)) return;
+#pragma unroll 1
+  for (uint32_t i = 0; i < (1u << 22); i++) {
+    if (mbar_try_wait_hint(bar, parity, WAIT_HINT_NS) || *abort_flag) return;
+  }
+  *abort_flag = 1;
+  if (status) atomicOr(status, ST_WAIT_EXPIRED);
+}
+
 constexpr int QT = 128;          // query rows per CTA
 constexpr int PT = 64;           // positions per tile
 constexpr float TAU = 5.0f;      // the reference max moves only when the true max exceeds it by this much
@@ -46,7 +79,8 @@ constexpr int SQ_BYTES = 2 * QT * 128;              // int8 Q: two K-halves of [
 constexpr int KST_BYTES = 2 * PT * 128 + PT * 16;   // one K (or V) stage: values + scales
 constexpr int VF_BYTES = 4 * PT * 128;              // f16 V: [4 dim chunks][64 positions][128 B]
 constexpr int P_BYTES = QT * 128;                   // f16 P: [128][64 positions]
-constexpr int DKF_BYTES = 8 * PT * 4;               // f32 K scales [8 blocks][64]
+constexpr int DKF_BYTES = 8 * PT * 4;               // f32 K scales [8 blocks][2 warpgroups][4 lanes tg][4 column groups][2]
+constexpr int OFS_BYTES = QT * 32;                  // operand of the offset MMA: 128 rows x 32 B of -128
 constexpr int OFF_Q = 0;
 constexpr int OFF_K = OFF_Q + SQ_BYTES;             // 2 stages (each padded to 18432 = 18 KB)
 constexpr int KST_PAD = 18432;
@@ -54,9 +88,10 @@ constexpr int OFF_V = OFF_K + 2 * KST_PAD;
 constexpr int OFF_VF = OFF_V + 2 * KST_PAD;
 constexpr int OFF_P = OFF_VF + 2 * VF_BYTES;
 constexpr int OFF_DKF = OFF_P + 2 * P_BYTES;
-constexpr int OFF_DQ = OFF_DKF + 2 * DKF_BYTES;     // f32 Q scales [8 blocks][128 rows] (a warp reads one block of 32 rows: no bank conflict)
-constexpr int OFF_XCH = OFF_DQ + QT * 8 * 4;        // row exchange between the two softmax warpgroups [tile parity][2][128] f32
-constexpr int OFF_BAR = OFF_XCH + 2 * 4 * QT * 4;   // room for four warpgroups
+constexpr int OFF_DQ = OFF_DKF + 2 * DKF_BYTES;     // f32 Q scales [8 blocks][4 warps q][8 lane groups g][4]: rows 32 q + g + 8 k
+constexpr int OFF_OFS = OFF_DQ + QT * 8 * 4;
+constexpr int OFF_XCH = OFF_OFS + OFS_BYTES;        // row exchange between the two softmax warpgroups [2][128] f32
+constexpr int OFF_BAR = OFF_XCH + 2 * QT * 4;
 constexpr int NBAR = 32;
 constexpr int OFF_MISC = OFF_BAR + NBAR * 8;        // tmem base address, abort flag
 constexpr int PF_SMEM_USED = OFF_MISC + 16;
@@ -75,27 +110,26 @@ enum {
   B_VFFULL = 9,   // [2]
   B_VFEMPTY = 11, // [2]
   B_DKEMPTY = 13, // [2]
-  B_SFULL = 15,   // [4]
-  B_SEMPTY = 19,  // [4]
+  B_SFULL = 15,   // [2] pairs of S slots
+  B_SEMPTY = 19,  // [2]
   B_PFULL = 23,   // [2]
   B_PEMPTY = 25,  // [2]
   B_ODONE = 27,
+  B_DKFULL = 28,  // [2]
 };
 
-#ifndef Q27B_PF_NWG
-#define Q27B_PF_NWG 2
-#endif
-constexpr int NWG = Q27B_PF_NWG;               // softmax warpgroups: each takes PT / NWG columns of a tile
-constexpr int WCOLS = PT / NWG;                // columns per softmax thread
+constexpr int NWG = 2;                         // softmax warpgroups: each takes PT / NWG columns of a tile
+constexpr int WCOLS = PT / NWG;                // columns per softmax warp
 constexpr int OCOLS = AD / NWG;                // columns of O per softmax thread (rescale, epilogue)
 constexpr int N_SOFTMAX_WARPS = 4 * NWG;
 constexpr int N_CONV_WARPS = 4;   // measured: 2 converter warps (and 162 registers for the softmax warps) lose 8 %
 constexpr int N_CONV_THREADS = N_CONV_WARPS * 32;
 constexpr int CONV_WARP0 = N_SOFTMAX_WARPS, TMA_WARP = CONV_WARP0 + N_CONV_WARPS, MMA_WARP = TMA_WARP + 1;
-constexpr int PF_THREADS = (MMA_WARP + 1) * 32;
+constexpr int PF_THREADS = (MMA_WARP + 3) * 32;  // whole warpgroups, for setmaxnreg
 constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t TM_O = 0, TM_S = 256;
 constexpr uint32_t IDESC_QK = umma_idesc(2, 1, 1, 0, 0, QT, PT);    // s32 += s8 * s8, both K-major, M128 N64
+constexpr uint32_t IDESC_OFS = umma_idesc(2, 1, 1, 0, 0, QT, 2 * PT);  // the offset of two S slots at once, M128 N128
 constexpr uint32_t IDESC_PV = umma_idesc(1, 0, 0, 0, 1, QT, AD);    // f32 += f16 * f16, B MN-major, M128 N256
 
 struct PrefillParams {
@@ -114,8 +148,20 @@ struct PrefillParams {
   float* xd;       // ... and one scale per 32 values, as f32(f16(d)) (q8_store, src/common.cuh:72-81)
 };
 
+// Powers of two that bring subnormal block sums (n * 2^-149) into the range of normal numbers; 2^(110 + 39) takes them out
+// again. An f16 scale times 2^110 stays below 2^126, a product with a block sum above 2^-63.
+constexpr float DK_SCALE = 0x1p110f, DQ_SCALE = 0x1p39f, OFS_SCALE = -0x1p-130f;  // OFS_SCALE: -2^19 * 2^-149
+
 // Barrier of the NWG threads' warps that share query rows 32q .. 32q+31.
 __device__ __forceinline__ void pair_sync(int q) { asm volatile("bar.sync %0, %1;" ::"r"(1 + q), "n"(32 * NWG) : "memory"); }
+
+// The same barrier with a vote: true for all of them when any thread says so.
+__device__ __forceinline__ bool pair_any(int q, bool x) {
+  uint32_t r;
+  asm volatile("{\n.reg .pred a, b;\nsetp.ne.u32 a, %1, 0;\nbar.red.or.pred b, %2, %3, a;\nselp.u32 %0, 1, 0, b;\n}\n"
+               : "=r"(r) : "r"((uint32_t)x), "r"(1 + q), "n"(32 * NWG) : "memory");
+  return r != 0;
+}
 
 // Quantises blocks [B0, B0 + NB) of one query row (256 floats at src, or zeros when src is null)
 // to int8 with an f32 scale per 32 dims (src/attn.cu:587-606: v = q * kq_scale, d = amax / 127,
@@ -161,10 +207,9 @@ __device__ __forceinline__ void quantise_q_row(const float* src, float kq_scale,
   }
 }
 
-// Multiplies OCOLS accumulator columns of this warp's 32 TMEM lanes by f. Rare (the reference max
-// of a row moves a few times per call), and deliberately not inlined: inlined, its 32 registers of
-// payload sit on top of the live state of the hot loop and push that loop into spills.
-__device__ __noinline__ void rescale_o(uint32_t taddr, float f) {
+// Multiplies OCOLS accumulator columns of this warp's 32 TMEM lanes by f. Rare: the reference max of a row moves a few
+// times per call.
+__device__ __forceinline__ void rescale_o(uint32_t taddr, float f) {
 #pragma unroll 1
   for (int c = 0; c < OCOLS / 32; c++) {
     uint32_t v[32];
@@ -174,6 +219,18 @@ __device__ __noinline__ void rescale_o(uint32_t taddr, float f) {
     for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * f);
     tmem_st32(taddr + c * 32, v);
   }
+}
+
+// The softmax warps hold rows g + 8 k (g = lane / 4, k = 0..3) in registers; this gives every thread the value of
+// row `lane` of its warp.
+__device__ __forceinline__ float row_of_lane(const float (&v)[4], int lane) {
+  float r = 0.f;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const float x = __shfl_sync(0xffffffffu, v[k], (lane & 7) * 4);
+    if ((lane >> 3) == k) r = x;
+  }
+  return r;
 }
 
 // Descriptors of the 32-byte k-block b of a K-major 128B-swizzled int8 tile made of two halves
@@ -196,10 +253,10 @@ prefill_i8_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_consta
   volatile int* abort_flag = (volatile int*)(sgen + OFF_MISC + 4);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // CTA order: the row tiles with the most positions first (src/attn.cu:567). tile_major: and that
-  // across all KV heads (block L = KV head L % nkvh of tile rank L / nkvh), which matters on a short prefix,
+  // CTA order: the query tiles with the most positions first (src/attn.cu:567). tile_major: and that
+  // across all heads (block L = head L % nqh of tile rank L / nqh), which matters on a short prefix,
   // where the tiles differ a lot in length and the longest tiles of the last heads would start last.
-  // Otherwise KV head by KV head (block L = tile rank L % n_tiles of KV head L / n_tiles), so that the CTAs
+  // Otherwise head by head (block L = tile rank L % n_tiles of head L / n_tiles), so that the CTAs
   // that run at the same time stream the same K/V rows and share them in L2 (measured: 7 % at 32k).
   // The unsplit CTAs (tiles >= ts) come first, then the pieces of the split tiles, split index slowest.
   int L = (int)blockIdx.x, z = 0, nsplit = 1, ntl = row_tiles(p.M) - p.ts, tile_base = p.ts;
@@ -242,10 +299,11 @@ prefill_i8_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_consta
       mbar_init(&bar[B_VFFULL + s], N_CONV_WARPS);
       mbar_init(&bar[B_VFEMPTY + s], 1);
       mbar_init(&bar[B_DKEMPTY + s], N_SOFTMAX_WARPS);
+      mbar_init(&bar[B_DKFULL + s], N_CONV_WARPS);
       mbar_init(&bar[B_PFULL + s], N_SOFTMAX_WARPS);
       mbar_init(&bar[B_PEMPTY + s], 1);
     }
-    for (int s = 0; s < 4; s++) {
+    for (int s = 0; s < 2; s++) {
       mbar_init(&bar[B_SFULL + s], 1);
       mbar_init(&bar[B_SEMPTY + s], N_SOFTMAX_WARPS);
     }
@@ -264,28 +322,29 @@ prefill_i8_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_consta
 
   if (warp < N_SOFTMAX_WARPS) {
     // ================================================================ softmax warps
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 176;");
     const int wg = warp >> 2, q = warp & 3;
-    const int r = q * 32 + lane;       // query row = TMEM lane
+    const int g = lane >> 2, tg = lane & 3;
+    const int r = q * 32 + lane;       // TMEM lane
     const int t = (row0 + r) / GQA, h = kh * GQA + (row0 + r) % GQA;
     const bool live = t < p.M;
-    float* xch = (float*)(sgen + OFF_XCH);
-    const float* dqs = (const float*)(sgen + OFF_DQ) + r;  // block b of this row at dqs[b * QT]
+    float* xch = (float*)(sgen + OFF_XCH) + q * 32 + 4 * g;  // rows g + 8 k of this warp, k = 0..3, side by side
+    const uint8_t* dqs = sgen + OFF_DQ + (q * 8 + g) * 16;     // ... and their Q scales of block b at dqs + 512 b
     {
       // this thread quantises 8 / NWG blocks of its row; the scales go through shared memory
       constexpr int NB = 8 / NWG;
       float dqh[NB];
       const float* src = live ? p.qn + ((size_t)t * p.nqh + h) * AD : nullptr;
-      if (NWG == 2) {
-        if (wg == 0) quantise_q_row<0, NB>(src, p.kq_scale, sgen + OFF_Q, r, dqh);
-        else quantise_q_row<NB, NB>(src, p.kq_scale, sgen + OFF_Q, r, dqh);
-      } else {
-        if (wg == 0) quantise_q_row<0, NB>(src, p.kq_scale, sgen + OFF_Q, r, dqh);
-        else if (wg == 1) quantise_q_row<NB, NB>(src, p.kq_scale, sgen + OFF_Q, r, dqh);
-        else if (wg == 2) quantise_q_row<(2 * NB) % 8, NB>(src, p.kq_scale, sgen + OFF_Q, r, dqh);
-        else quantise_q_row<(3 * NB) % 8, NB>(src, p.kq_scale, sgen + OFF_Q, r, dqh);
-      }
+      if (wg == 0) quantise_q_row<0, NB>(src, p.kq_scale, sgen + OFF_Q, r, dqh);
+      else quantise_q_row<NB, NB>(src, p.kq_scale, sgen + OFF_Q, r, dqh);
 #pragma unroll
-      for (int i = 0; i < NB; i++) *(float*)(sgen + OFF_DQ + ((NB * wg + i) * QT + r) * 4) = dqh[i];
+      for (int i = 0; i < NB; i++)
+        *(float*)(sgen + OFF_DQ + (((NB * wg + i) * 4 + q) * 8 + (lane & 7)) * 16 + (lane >> 3) * 4) = dqh[i] * DQ_SCALE;
+      if (wg == 0) {
+        const uint4 w = make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u);
+        *(uint4*)(sgen + OFF_OFS + r * 32) = w;
+        *(uint4*)(sgen + OFF_OFS + r * 32 + 16) = w;
+      }
       fence_proxy_async();
       pair_sync(q);
       __syncwarp();
@@ -293,195 +352,239 @@ prefill_i8_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_consta
     }
 
     const uint32_t tlane = tmem + ((uint32_t)(q * 32) << 16);
-    const int limit = pos0 + t + 1;    // positions < limit are visible
-    const int col0 = wg * WCOLS;       // this thread's positions of a tile: col0 .. col0 + WCOLS - 1
-    float m_run = M_INIT, m_ref = M_INIT;
-    uint64_t l2 = pack2(0.f, 0.f);
+    const int col0 = wg * WCOLS;       // this warp's positions of a tile: col0 .. col0 + WCOLS - 1
+    int limit[4];                      // positions < limit[k] are visible to row g + 8 k
+#pragma unroll
+    for (int k = 0; k < 4; k++) limit[k] = pos0 + (row0 + q * 32 + g + 8 * k) / GQA + 1 - col0 - 2 * tg;
+    float m_ref[4];
+    uint64_t l2[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      m_ref[k] = M_INIT;
+      l2[k] = pack2(0.f, 0.f);
+    }
     const uint64_t log2e2 = pack2(LOG2E, LOG2E);
+    const uint64_t ofs2 = pack2(OFS_SCALE, OFS_SCALE);
 
 #pragma unroll 1
     for (int j = 0; j < nt; j++) {
-      const int pb = j & 1, ph = (j >> 1) & 1;
+      const int pb = j & 1;
       const int p_tile = (it0 + j) * PT;
-      mbar_wait(&bar[B_VFFULL + pb], ph, abort_flag, p.status);  // K scale table of this tile is ready
-      const uint8_t* dkf = sgen + OFF_DKF + pb * DKF_BYTES;
-      uint64_t s2[WCOLS / 2];
+      const uint8_t* dkf = sgen + OFF_DKF + pb * DKF_BYTES + wg * 128 + tg * 32;
+      // s2[k][i]: row g + 8 k, positions col0 + 8 i + 2 tg, + 1
+      uint64_t s2[4][4];
 #pragma unroll
-      for (int i = 0; i < WCOLS / 2; i++) s2[i] = pack2(0.f, 0.f);
+      for (int k = 0; k < 4; k++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) s2[k][i] = pack2(0.f, 0.f);
 #pragma unroll
       for (int b = 0; b < 8; b++) {
         const int slot = b & 3;
-#ifdef Q27B_PF_COMMIT_EACH
-        mbar_wait(&bar[B_SFULL + slot], (b >> 2) & 1, abort_flag, p.status);
-#else
-        // (blocks are committed in pairs: the barrier of the pair's second slot covers both)
-        mbar_wait(&bar[B_SFULL + (slot | 1)], (b >> 2) & 1, abort_flag, p.status);
-#endif
-        tc_fence_after();
-        // The accumulators come in two halves of 16 columns: 16 registers fewer are live at a time
-        // than with one 32-column load, and this kernel runs at its register limit.
-        const float dqv = dqs[b * QT];  // this row's Q scale of block b (shared memory: eight registers fewer)
-        const uint64_t dqb = pack2(dqv, dqv);
+        if ((b & 1) == 0) {
+          pf_wait(&bar[B_SFULL + (slot >> 1)], (b >> 2) & 1, abort_flag, p.status);
+          tc_fence_after();
+        }
+        const ulonglong2 dk01 = *(const ulonglong2*)(dkf + b * 256), dk23 = *(const ulonglong2*)(dkf + b * 256 + 16);
+        const uint64_t dk[4] = {dk01.x, dk01.y, dk23.x, dk23.y};
+        const float4 dq4 = *(const float4*)(dqs + b * 512);
+        const float dq[4] = {dq4.x, dq4.y, dq4.z, dq4.w};
+        uint64_t dc[4];
 #pragma unroll
-        for (int hf = 0; hf < WCOLS / 16; hf++) {
+        for (int i = 0; i < 4; i++) dc[i] = mul2(dk[i], ofs2);
+#pragma unroll
+        for (int hf = 0; hf < 2; hf++) {  // TMEM lanes 16 hf .. 16 hf + 15 of this warp: rows g + 16 hf and g + 8 + 16 hf
           uint32_t v[16];
-          tmem_ld16(tlane + TM_S + slot * PT + col0 + 16 * hf, v);
+          tmem_ld16x256(tlane + ((uint32_t)(16 * hf) << 16) + TM_S + slot * PT + col0, v);
           tc_wait_ld();
-          if (hf == WCOLS / 16 - 1) {
+          if (hf == 1 && (b & 1)) {
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&bar[B_SEMPTY + slot]);  // the slot is in registers: it can be overwritten
+            if (lane == 0) mbar_arrive(&bar[B_SEMPTY + (slot >> 1)]);  // the pair is in registers: it can be overwritten
           }
-          const ulonglong2* dk2 = (const ulonglong2*)(dkf + (b * PT + col0 + 16 * hf) * 4);
 #pragma unroll
-          for (int i = 0; i < 4; i++) {
-            const ulonglong2 dk = dk2[i];  // K scales of positions 4i .. 4i+3 (block b)
-            // int32 -> f32 is exact here (|sum| <= 32 * 127 * 127 < 2^24)
-            const uint64_t f0 = pack2(__int2float_rn((int)v[4 * i]), __int2float_rn((int)v[4 * i + 1]));
-            const uint64_t f1 = pack2(__int2float_rn((int)v[4 * i + 2]), __int2float_rn((int)v[4 * i + 3]));
-            s2[8 * hf + 2 * i] = fma2(mul2(dqb, dk.x), f0, s2[8 * hf + 2 * i]);
-            s2[8 * hf + 2 * i + 1] = fma2(mul2(dqb, dk.y), f1, s2[8 * hf + 2 * i + 1]);
+          for (int e = 0; e < 2; e++) {
+            const int k = 2 * hf + e;
+            const uint64_t dqb = pack2(dq[k], dq[k]);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+              const uint64_t x = pack2(__uint_as_float(v[4 * i + 2 * e]), __uint_as_float(v[4 * i + 2 * e + 1]));
+              s2[k][i] = fma2(dqb, fma2(dk[i], x, dc[i]), s2[k][i]);
+            }
           }
         }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar[B_DKEMPTY + pb]);
 
-      // causal mask (only tiles that reach past the first row's limit need it) and this thread's max
-      float s[WCOLS];
+      // causal mask (only tiles that reach past the first row's limit need it) and the rows' maxima
+      float s[4][8], mt[4];
 #pragma unroll
-      for (int i = 0; i < WCOLS / 2; i++) unpack2(s2[i], s[2 * i], s[2 * i + 1]);
-      float mt = -INFINITY;
+      for (int k = 0; k < 4; k++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) unpack2(s2[k][i], s[k][2 * i], s[k][2 * i + 1]);
       if (p_tile + PT > pos0 + t0 + 1) {
 #pragma unroll
-        for (int i = 0; i < WCOLS; i++) {
-          if (p_tile + col0 + i >= limit) s[i] = -INFINITY;
-          mt = fmaxf(mt, s[i]);
-        }
-      } else {
+        for (int k = 0; k < 4; k++)
 #pragma unroll
-        for (int i = 0; i < WCOLS; i++) mt = fmaxf(mt, s[i]);
+          for (int i = 0; i < 8; i++)
+            if (p_tile + 8 * (i >> 1) + (i & 1) >= limit[k]) s[k][i] = -INFINITY;
       }
-      // row maximum over the NWG threads of the row; the buffer alternates with the tile so that a
-      // fast thread cannot overwrite what a partner has not read yet
-      xch[(pb * NWG + wg) * QT + r] = mt;
-      pair_sync(q);
+      // The reference maxima move when some score of the tile exceeds its row's by more than TAU (and on the first
+      // tile). Whether one does is all that the two warps of the rows have to agree on in the common case: one
+      // barrier that ORs their votes.
+      bool want = false;
 #pragma unroll
-      for (int o = 1; o < NWG; o++) mt = fmaxf(mt, xch[(pb * NWG + ((wg + o) % NWG)) * QT + r]);
-      m_run = fmaxf(m_run, mt);
-
-      // Move the reference max when the true max has run away from it (and on the first tile). All
-      // threads of a row hold the same m_run and m_ref, so all their warps take the same branch.
-      const bool want = m_run > m_ref + TAU;
-      if (__any_sync(0xffffffffu, want)) {
-        const float f = ex2((m_ref - m_run) * LOG2E);  // 0 on the first move (m_ref = -1e30)
-        m_ref = m_run;
-        l2 = mul2(l2, pack2(f, f));
+      for (int k = 0; k < 4; k++) {
+        mt[k] = fmaxf(fmaxf(fmaxf(s[k][0], s[k][1]), fmaxf(s[k][2], s[k][3])), fmaxf(fmaxf(s[k][4], s[k][5]), fmaxf(s[k][6], s[k][7])));
+        want |= mt[k] > m_ref[k] + TAU;
+      }
+      if (pair_any(q, want)) {
+        float f[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          mt[k] = fmaxf(mt[k], __shfl_xor_sync(0xffffffffu, mt[k], 1));
+          mt[k] = fmaxf(mt[k], __shfl_xor_sync(0xffffffffu, mt[k], 2));
+        }
+        xch[wg * QT + tg] = tg == 0 ? mt[0] : tg == 1 ? mt[1] : tg == 2 ? mt[2] : mt[3];
+        pair_sync(q);
+        const float4 o4 = *(const float4*)(xch + (wg ^ 1) * QT);
+        pair_sync(q);  // both have read: the next move may write
+        const float ot[4] = {o4.x, o4.y, o4.z, o4.w};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const float m = fmaxf(m_ref[k], fmaxf(mt[k], ot[k]));
+          f[k] = ex2((m_ref[k] - m) * LOG2E);  // 0 on the first move (m_ref = -1e30)
+          m_ref[k] = m;
+          l2[k] = mul2(l2[k], pack2(f[k], f[k]));
+        }
         if (j > 0) {
           // O holds the sum of tiles < j once the P V of tile j-1 has completed. This warp rescales
           // columns OCOLS wg .. OCOLS wg + OCOLS - 1 of its 32 rows.
-          mbar_wait(&bar[B_PEMPTY + ((j - 1) & 1)], ((j - 1) >> 1) & 1, abort_flag, p.status);
+          pf_wait(&bar[B_PEMPTY + ((j - 1) & 1)], ((j - 1) >> 1) & 1, abort_flag, p.status);
           tc_fence_after();
-          rescale_o(tlane + TM_O + wg * OCOLS, f);
+          rescale_o(tlane + TM_O + wg * OCOLS, row_of_lane(f, lane));
           tc_wait_st();
           tc_fence_before();
         }
       }
 
-      // P = exp(s - m_ref): f32 row sum, f16 part of the tile for the P V MMA (WCOLS / 8 chunks of the row)
-      mbar_wait(&bar[B_PEMPTY + pb], ph ^ 1, abort_flag, p.status);
-      uint8_t* sP = sgen + OFF_P + pb * P_BYTES;
-      const float nmb = -m_ref * LOG2E;
-      const uint64_t nmb2 = pack2(nmb, nmb);
+      // P = exp(s - m_ref): f32 row sums, f16 part of the tile for the P V MMA
+      uint8_t* sP = sgen + OFF_P + pb * P_BYTES + (q * 32 + g) * 128 + 4 * tg;
 #pragma unroll
-      for (int c = 0; c < WCOLS / 8; c++) {
-        uint32_t w[4];
+      for (int k = 0; k < 4; k++) {
+        const float nmb = -m_ref[k] * LOG2E;
+        const uint64_t nmb2 = pack2(nmb, nmb);
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
+        for (int i = 0; i < 4; i++) {
           float a0, a1;
-          unpack2(fma2(pack2(s[c * 8 + 2 * k], s[c * 8 + 2 * k + 1]), log2e2, nmb2), a0, a1);
+          unpack2(fma2(pack2(s[k][2 * i], s[k][2 * i + 1]), log2e2, nmb2), a0, a1);
           const float e0 = ex2(a0), e1 = ex2(a1);
-          l2 = add2(l2, pack2(e0, e1));
-          w[k] = pack_h2(e0, e1);
+          l2[k] = add2(l2[k], pack2(e0, e1));
+          *(uint32_t*)(sP + k * 1024 + (((4 * wg + i) ^ g) << 4)) = pack_h2(e0, e1);
         }
-        *(uint4*)(sP + swz128(r, (WCOLS / 8) * wg + c)) = make_uint4(w[0], w[1], w[2], w[3]);
       }
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar[B_PFULL + pb]);
     }
 
-    // ---- epilogue: O / l * sigmoid(gate), or the unnormalised partial of this split; this thread
-    // writes columns OCOLS wg .. OCOLS wg + OCOLS - 1 of its row
-    float la, lb;
-    unpack2(l2, la, lb);
-    float l = la + lb;
-    xch[((nt & 1) * NWG + wg) * QT + r] = l;
-    pair_sync(q);
+    // ---- epilogue: O / l * sigmoid(gate), or the unnormalised partial of this split; this warp
+    // writes columns OCOLS wg .. OCOLS wg + OCOLS - 1 of its rows
+    float l4[4];
 #pragma unroll
-    for (int o = 1; o < NWG; o++) l += xch[((nt & 1) * NWG + ((wg + o) % NWG)) * QT + r];
-    mbar_wait(&bar[B_ODONE], 0, abort_flag, p.status);
+    for (int k = 0; k < 4; k++) {
+      float la, lb;
+      unpack2(l2[k], la, lb);
+      l4[k] = la + lb;
+      l4[k] += __shfl_xor_sync(0xffffffffu, l4[k], 1);
+      l4[k] += __shfl_xor_sync(0xffffffffu, l4[k], 2);
+    }
+    xch[wg * QT + tg] = tg == 0 ? l4[0] : tg == 1 ? l4[1] : tg == 2 ? l4[2] : l4[3];
+    pair_sync(q);
+    {
+      const float4 o4 = *(const float4*)(xch + (wg ^ 1) * QT);
+      l4[0] += o4.x; l4[1] += o4.y; l4[2] += o4.z; l4[3] += o4.w;
+    }
+    const float l = row_of_lane(l4, lane), m_row = row_of_lane(m_ref, lane);
+    pf_wait(&bar[B_ODONE], 0, abort_flag, p.status);
     tc_fence_after();
     const float inv_l = 1.0f / l;
-    float* po = nsplit > 1 ? p.part + (((size_t)z * p.Ms + t) * p.nqh + h) * PROW : nullptr;
-    if (live && po && wg == 0) {
-      po[0] = m_ref;
-      po[1] = l;
+    if (nsplit > 1 && wg == 0) {
+      const int t = (row0 + r) / GQA;
+      if (t < p.M) *(float2*)(p.part + (((size_t)z * p.Ms + t) * p.nqh + kh * GQA + (row0 + r) % GQA) * PROW) = make_float2(m_row, l);
     }
+    // 32 columns at a time through shared memory (the f16 V buffers are free now): TMEM gives a thread a row, and a row
+    // per thread would touch 32 lines with every load of the gate and every store; read back, eight lanes share 128
+    // contiguous bytes of a row (2,048 tokens without a prefix 213 -> 201 us, 16 behind 30,000 58 -> 52).
+    uint8_t* stage = sgen + OFF_VF + warp * 4096;
 #pragma unroll 1
     for (int c = 0; c < OCOLS / 32; c++) {
       const int d0 = wg * OCOLS + c * 32;
-      uint32_t v[32];
-      tmem_ld32(tlane + TM_O + d0, v);
-      tc_wait_ld();
-      if (!live) continue;
-      if (po) {
+      float4 gate[8];
+      if (nsplit == 1) {
 #pragma unroll
-        for (int i = 0; i < 32; i += 2)
-          *(float2*)(po + 2 + d0 + i) = make_float2(__uint_as_float(v[i]), __uint_as_float(v[i + 1]));
-      } else {
-        const float* gt = p.qg + ((size_t)t * p.nqh + h) * 512 + 256 + d0;
-        float* dst = p.xq ? nullptr : p.o + ((size_t)t * p.nqh + h) * AD + d0;
-        float amax = 0.f;
-#pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-          const float4 gg = *(const float4*)(gt + i);
-          float4 y;
-          y.x = (__uint_as_float(v[i]) * inv_l) * (1.0f / (1.0f + __expf(-gg.x)));
-          y.y = (__uint_as_float(v[i + 1]) * inv_l) * (1.0f / (1.0f + __expf(-gg.y)));
-          y.z = (__uint_as_float(v[i + 2]) * inv_l) * (1.0f / (1.0f + __expf(-gg.z)));
-          y.w = (__uint_as_float(v[i + 3]) * inv_l) * (1.0f / (1.0f + __expf(-gg.w)));
-          if (dst) {
-            *(float4*)(dst + i) = y;
-          } else {  // keep the values for the q8_1 block below (these 32 columns are exactly one block)
-            v[i] = __float_as_uint(y.x); v[i + 1] = __float_as_uint(y.y);
-            v[i + 2] = __float_as_uint(y.z); v[i + 3] = __float_as_uint(y.w);
-            amax = fmaxf(amax, fmaxf(fmaxf(fabsf(y.x), fabsf(y.y)), fmaxf(fabsf(y.z), fabsf(y.w))));
-          }
-        }
-        if (!dst) {
-          // q8_1 as the reference's quantize_q8_1 / q8_store (src/common.cuh:72-81): d = amax / 127,
-          // q = round(y / d) (half away from zero), the scale leaves as f32(f16(d)); IEEE division
-          const float dd = __fdiv_rn(amax, 127.0f);
-          const size_t oi = ((size_t)t * p.nqh + h) * AD + d0;
-          uint32_t w[8];
-#pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            uint32_t b[4];
-#pragma unroll
-            for (int k = 0; k < 4; k++)
-              b[k] = amax == 0.0f ? 0u : (uint32_t)(uint8_t)(int8_t)roundf(__fdiv_rn(__uint_as_float(v[i + k]), dd));
-            w[i / 4] = b[0] | (b[1] << 8) | (b[2] << 16) | (b[3] << 24);
-          }
-          *(uint4*)(p.xq + oi) = make_uint4(w[0], w[1], w[2], w[3]);
-          *(uint4*)(p.xq + oi + 16) = make_uint4(w[4], w[5], w[6], w[7]);
-          p.xd[oi / 32] = __half2float(__float2half_rn(dd));
+        for (int i = 0; i < 8; i++) {
+          const int gr = row0 + q * 32 + 4 * i + (lane >> 3), t = gr / GQA;
+          if (t < p.M) gate[i] = *(const float4*)(p.qg + ((size_t)t * p.nqh + kh * GQA + gr % GQA) * 512 + 256 + d0 + 4 * (lane & 7));
         }
       }
+      {
+        uint32_t v[32];
+        tmem_ld32(tlane + TM_O + d0, v);
+        tc_wait_ld();
+        const float f = nsplit > 1 ? 1.f : inv_l;
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+          *(float4*)(stage + swz128(lane, i)) = make_float4(__uint_as_float(v[4 * i]) * f, __uint_as_float(v[4 * i + 1]) * f,
+                                                            __uint_as_float(v[4 * i + 2]) * f, __uint_as_float(v[4 * i + 3]) * f);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const int rr = 4 * i + (lane >> 3), gr = row0 + q * 32 + rr, t = gr / GQA;
+        const size_t th = (size_t)t * p.nqh + kh * GQA + gr % GQA;
+        const int d = d0 + 4 * (lane & 7);
+        const bool live = t < p.M;
+        float4 y = *(const float4*)(stage + swz128(rr, lane & 7));
+        if (nsplit > 1) {
+          if (live) {
+            float* po = p.part + ((size_t)z * p.Ms * p.nqh + th) * PROW + 2 + d;
+            *(float2*)po = make_float2(y.x, y.y);
+            *(float2*)(po + 2) = make_float2(y.z, y.w);
+          }
+          continue;
+        }
+        if (live) {
+          const float4 gg = gate[i];
+          y.x *= 1.0f / (1.0f + __expf(-gg.x));
+          y.y *= 1.0f / (1.0f + __expf(-gg.y));
+          y.z *= 1.0f / (1.0f + __expf(-gg.z));
+          y.w *= 1.0f / (1.0f + __expf(-gg.w));
+          if (!p.xq) *(float4*)(p.o + th * AD + d) = y;
+        }
+        if (p.xq) {
+          // q8_1 as the reference's quantize_q8_1 / q8_store (src/common.cuh:72-81): d = amax / 127, q = round(y / d)
+          // (half away from zero), the scale leaves as f32(f16(d)); IEEE division. These 32 columns are one block.
+          float amax = fmaxf(fmaxf(fabsf(y.x), fabsf(y.y)), fmaxf(fabsf(y.z), fabsf(y.w)));
+#pragma unroll
+          for (int o = 1; o <= 4; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+          const float dd = __fdiv_rn(amax, 127.0f), yy[4] = {y.x, y.y, y.z, y.w};
+          uint32_t w = 0;
+#pragma unroll
+          for (int k = 0; k < 4; k++)
+            w |= (amax == 0.0f ? 0u : (uint32_t)(uint8_t)(int8_t)roundf(__fdiv_rn(yy[k], dd))) << (8 * k);
+          if (live) {
+            *(uint32_t*)(p.xq + th * AD + d) = w;
+            if ((lane & 7) == 0) p.xd[(th * AD + d) / 32] = __half2float(__float2half_rn(dd));
+          }
+        }
+      }
+      __syncwarp();
     }
     tc_fence_before();
   } else if (warp < TMA_WARP) {
     // ================================================================ converter warps
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
     const int ct = tid - CONV_WARP0 * 32;
     static_assert(N_CONV_THREADS == 128, "the item mapping below is for 128 converter threads");
     const int cv_row0 = (2 * (ct >> 5)) ^ (5 * ((ct >> 2) & 1)), cv_c16 = (ct & 3) + 4 * ((ct >> 3) & 3);
@@ -490,12 +593,36 @@ prefill_i8_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_consta
     const uint32_t cv_dst = (cv_c16 >> 2) * (PT * 128) + swz128(cv_row0, 2 * (cv_c16 & 3));
     for (int j = 0; j < nt; j++) {
       const int pb = j & 1, ph = (j >> 1) & 1;
-      mbar_wait(&bar[B_VFULL + pb], ph, abort_flag, p.status);
-      mbar_wait(&bar[B_KFULL + pb], ph, abort_flag, p.status);
-      mbar_wait(&bar[B_VFEMPTY + pb], ph ^ 1, abort_flag, p.status);
-      mbar_wait(&bar[B_DKEMPTY + pb], ph ^ 1, abort_flag, p.status);
       const uint8_t* vst = sgen + OFF_V + pb * KST_PAD;
       const uint8_t* kst = sgen + OFF_K + pb * KST_PAD;
+      // The scale table first: Q K^T of this tile needs it, while V has to wait for the buffer that the P V of two tiles
+      // back reads.
+      pf_wait(&bar[B_KFULL + pb], ph, abort_flag, p.status);
+      pf_wait(&bar[B_DKEMPTY + pb], ph ^ 1, abort_flag, p.status);
+      // K scales f16 [64][8] -> f32 [8][64]
+      {
+        float* dkf = (float*)(sgen + OFF_DKF + pb * DKF_BYTES);
+#pragma unroll
+        for (int u = ct; u < 128; u += N_CONV_THREADS) {
+          const int row = u >> 1, b0 = (u & 1) * 4;
+          const uint2 sc = *(const uint2*)(kst + 2 * PT * 128 + row * 16 + b0 * 2);
+          const __half2 s01 = u32_as_h2(sc.x), s23 = u32_as_h2(sc.y);
+          const float d4[4] = {__low2float(s01), __high2float(s01), __low2float(s23), __high2float(s23)};
+          // An infinite scale (a K value above 8.3 million) counts as the largest finite one: the offset of the block sums
+          // must cancel, inf - inf would not.
+          // position row = 32 wg + 8 i + 2 tg + e -> [block][wg][tg][i][e]
+          float* dst = dkf + (row >> 5) * 32 + ((row >> 1) & 3) * 8 + ((row >> 3) & 3) * 2 + (row & 1);
+#pragma unroll
+          for (int i = 0; i < 4; i++) dst[(b0 + i) * PT] = (d4[i] == INFINITY ? 65504.f : d4[i]) * DK_SCALE;
+        }
+      }
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&bar[B_DKFULL + pb]);
+        mbar_arrive(&bar[B_KEMPTY + pb]);
+      }
+      pf_wait(&bar[B_VFULL + pb], ph, abort_flag, p.status);
+      pf_wait(&bar[B_VFEMPTY + pb], ph ^ 1, abort_flag, p.status);
       uint8_t* vf = sgen + OFF_VF + pb * VF_BYTES;
       // V: 64 rows x 16 chunks of 16 int8 -> 16 f16 (one rounding of q * d, as src/attn.cu:59-76).
       // Item = (row, 16-dim chunk); eight neighbouring lanes take 4 chunks of rows rho and rho ^ 5,
@@ -532,29 +659,16 @@ prefill_i8_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_consta
           *(uint4*)(dst + (cv_dst ^ 16u)) = make_uint4(o[4], o[5], o[6], o[7]);
         }
       }
-      // K scales f16 [64][8] -> f32 [8][64]
-      {
-        float* dkf = (float*)(sgen + OFF_DKF + pb * DKF_BYTES);
-#pragma unroll
-        for (int u = ct; u < 128; u += N_CONV_THREADS) {
-          const int row = u >> 1, b0 = (u & 1) * 4;
-          const uint2 sc = *(const uint2*)(kst + 2 * PT * 128 + row * 16 + b0 * 2);
-          const __half2 s01 = u32_as_h2(sc.x), s23 = u32_as_h2(sc.y);
-          dkf[(b0 + 0) * PT + row] = __low2float(s01);
-          dkf[(b0 + 1) * PT + row] = __high2float(s01);
-          dkf[(b0 + 2) * PT + row] = __low2float(s23);
-          dkf[(b0 + 3) * PT + row] = __high2float(s23);
-        }
-      }
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(&bar[B_VFFULL + pb]);
         mbar_arrive(&bar[B_VEMPTY + pb]);
-        mbar_arrive(&bar[B_KEMPTY + pb]);
       }
     }
-  } else if (warp == TMA_WARP) {
+  } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    if (warp == TMA_WARP) {
     // ================================================================ TMA producer
     if (lane == 0) {
       tma_prefetch_desc(&tm_kv);
@@ -566,27 +680,28 @@ prefill_i8_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_consta
         const int row = kh * p.n_ctx + (it0 + j) * PT;
         uint8_t* kst = sgen + OFF_K + pb * KST_PAD;
         uint8_t* vst = sgen + OFF_V + pb * KST_PAD;
-        mbar_wait(&bar[B_KEMPTY + pb], ph ^ 1, abort_flag, p.status);
+        pf_wait(&bar[B_KEMPTY + pb], ph ^ 1, abort_flag, p.status);
         mbar_expect_tx(&bar[B_KFULL + pb], KST_BYTES);
         tma_load_2d(kst, &tm_kv, 0, row, &bar[B_KFULL + pb]);
         tma_load_2d(kst + PT * 128, &tm_kv, 128, row, &bar[B_KFULL + pb]);
         tma_load_2d(kst + 2 * PT * 128, &tm_ks, 0, row, &bar[B_KFULL + pb]);
-        mbar_wait(&bar[B_VEMPTY + pb], ph ^ 1, abort_flag, p.status);
+        pf_wait(&bar[B_VEMPTY + pb], ph ^ 1, abort_flag, p.status);
         mbar_expect_tx(&bar[B_VFULL + pb], KST_BYTES);
         tma_load_2d(vst, &tm_vv, 0, row, &bar[B_VFULL + pb]);
         tma_load_2d(vst + PT * 128, &tm_vv, 128, row, &bar[B_VFULL + pb]);
         tma_load_2d(vst + 2 * PT * 128, &tm_vs, 0, row, &bar[B_VFULL + pb]);
       }
     }
-  } else {
+  } else if (warp == MMA_WARP) {
     // ================================================================ MMA issuer
     if (lane == 0) {
-      mbar_wait(&bar[B_QFULL], 0, abort_flag, p.status);
+      pf_wait(&bar[B_QFULL], 0, abort_flag, p.status);
       tc_fence_after();
+      const uint64_t desc_ofs = umma_desc_plain(sbase + OFF_OFS, 128, 256);
       auto issue_pv = [&](int jj) {
         const int pb = jj & 1, ph = (jj >> 1) & 1;
-        mbar_wait(&bar[B_PFULL + pb], ph, abort_flag, p.status);
-        mbar_wait(&bar[B_VFFULL + pb], ph, abort_flag, p.status);
+        pf_wait(&bar[B_PFULL + pb], ph, abort_flag, p.status);
+        pf_wait(&bar[B_VFFULL + pb], ph, abort_flag, p.status);
         tc_fence_after();
 #pragma unroll
         for (int kk = 0; kk < PT / 16; kk++) {
@@ -599,29 +714,27 @@ prefill_i8_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_consta
       };
       for (int j = 0; j < nt; j++) {
         const int pb = j & 1, ph = (j >> 1) & 1;
-        mbar_wait(&bar[B_KFULL + pb], ph, abort_flag, p.status);
+        pf_wait(&bar[B_KFULL + pb], ph, abort_flag, p.status);
+        pf_wait(&bar[B_DKFULL + pb], ph, abort_flag, p.status);  // the softmax warps find the K scale table behind the first commit
         tc_fence_after();
 #pragma unroll
         for (int b = 0; b < 8; b++) {
           const int slot = b & 3;
-          mbar_wait(&bar[B_SEMPTY + slot], ((b >> 2) & 1) ^ 1, abort_flag, p.status);
-          tc_fence_after();
+          if ((b & 1) == 0) {
+            pf_wait(&bar[B_SEMPTY + (slot >> 1)], ((b >> 2) & 1) ^ 1, abort_flag, p.status);
+            tc_fence_after();
+            tc_mma_i8(tmem + TM_S + slot * PT, desc_ofs, desc_ofs, IDESC_OFS, 0u);
+          }
           tc_mma_i8(tmem + TM_S + slot * PT, desc_kblock(sbase + OFF_Q, QT, b),
-                    desc_kblock(sbase + OFF_K + pb * KST_PAD, PT, b), IDESC_QK, 0u);
-#ifdef Q27B_PF_COMMIT_EACH
-          tc_commit(&bar[B_SFULL + slot]);
-#else
-          // One commit per two blocks: an MMA followed by its own commit costs the issuing thread the better
-          // part of a thousand cycles (measured on the decode kernel with P V on tcgen05), eight of them per
-          // tile were most of a tile's time here.
-          if (b & 1) tc_commit(&bar[B_SFULL + slot]);
-#endif
+                    desc_kblock(sbase + OFF_K + pb * KST_PAD, PT, b), IDESC_QK, 1u);
+          if (b & 1) tc_commit(&bar[B_SFULL + (slot >> 1)]);
         }
         tc_commit(&bar[B_KEMPTY + pb]);
         if (j >= 1) issue_pv(j - 1);
       }
       issue_pv(nt - 1);
       tc_commit(&bar[B_ODONE]);
+    }
     }
   }
 
@@ -692,13 +805,13 @@ prefill_qk_debug_kernel(const __grid_constant__ CUtensorMap tm_kv, const QkDebug
     mbar_expect_tx(&bar[0], 2 * PT * 128);
     tma_load_2d(sgen + DBG_OFF_K, &tm_kv, 0, p.row0, &bar[0]);
     tma_load_2d(sgen + DBG_OFF_K + PT * 128, &tm_kv, 128, p.row0, &bar[0]);
-    mbar_wait(&bar[0], 0, abort_flag, p.status);
+    pf_wait(&bar[0], 0, abort_flag, p.status);
     tc_fence_after();
     for (int b = 0; b < 8; b++)
       tc_mma_i8(tmem + b * PT, desc_kblock(sbase, QT, b), desc_kblock(sbase + DBG_OFF_K, PT, b), IDESC_QK, 0u);
     tc_commit(&bar[1]);
   }
-  mbar_wait(&bar[1], 0, abort_flag, p.status);
+  pf_wait(&bar[1], 0, abort_flag, p.status);
   tc_fence_after();
   const uint32_t tlane = tmem + ((uint32_t)(warp * 32) << 16);
   for (int b = 0; b < 8; b++)

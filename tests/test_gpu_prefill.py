@@ -354,3 +354,29 @@ def test_prefill_f16_qk_on_q8_cache(q27, orc, pos0, M, depth_hint):
     ref = orc.attn_ref(qn, qg, kc_ref, vc_ref, pos0, SCALE, nkvh, n_ctx, q8=True)
     assert_close(o.cpu().numpy(), ref, "f16-QK prefill on q8_0 pos0=%d M=%d" % (pos0, M))
     assert q27.device_status() == 0
+
+
+@pytest.mark.parametrize("qs,ks", [(1e-4, 1e4), (1e4, 1e-4), (1e-6, 1e6), (1e-20, 1.0), (30.0, 1.0)])
+def test_prefill_i8_magnitudes(q27, orc, qs, ks):
+    """The int8 kernel reads block sums as subnormal floats and moves powers of two between the Q and the K scales: the
+    ends of their ranges (K scales from f16 subnormals to near the largest f16, tiny Q) against the oracle, and scores
+    large enough to move the reference maxima on most tiles (qs = 30). Tolerance as everywhere: the arithmetic is exact up
+    to f32 rounding."""
+    from qwen27_engine_b200 import synth
+    pos0, M, nkvh = 333, 40, 1
+    nqh, n = nkvh * GQA, pos0 + M
+    n_ctx = n + 9
+    qn = synth.normal(synth.SEED_Q, (M, nqh, AD)) * np.float32(qs)
+    qg = np.zeros((M, nqh, 512), np.float32)
+    qg[..., 256:] = synth.normal(synth.SEED_GATE, (M, nqh, AD))
+    kc_ref, vc_ref = orc.fill_cache(synth.normal(synth.SEED_K, (nkvh, n, AD)) * np.float32(ks),
+                                    synth.normal(synth.SEED_V, (nkvh, n, AD)), n_ctx)
+    o = torch.full((M, nqh, AD), float("nan"), device="cuda")
+    q27.attn_prefill(dev(qn), dev(qg), poisoned_cache(q27, kc_ref, nkvh, n_ctx, n), poisoned_cache(q27, vc_ref, nkvh, n_ctx, n),
+                     o, pos_tensor(pos0), M, SCALE, nqh, nkvh, n_ctx)
+    torch.cuda.synchronize()
+    ref = orc.attn_prefill_i8(qn, qg, kc_ref, vc_ref, pos0, SCALE, nkvh, n_ctx)
+    # P and V are rounded to f16 (2^-11 of a value); with few positions carrying a row (qs = 30) the outputs are of the
+    # size of V itself, so the bound is relative to their RMS
+    assert_close(o.cpu().numpy(), ref, "qs=%g ks=%g" % (qs, ks), abs_tol=1e-2 * float(np.sqrt((ref.astype(np.float64) ** 2).mean())))
+    assert q27.device_status() == 0
