@@ -30,9 +30,9 @@
 // TMEM: columns 0-255 O (f32), 256-511 four S slots of 64 columns (s32).
 //
 // What bounds it: the SIMT lanes of the softmax warps, two warps on each quarter of the SM, which share rows and so
-// run through the same phases together. Per tile (clock stamps, 148,000 positions): 4,300 cycles at first, of them
-// 2,500 in the scale loop, 680 for the row maxima, 740 for exp and P, 450 waiting for barriers that had long
-// completed. What was changed (2,048 tokens behind 148,000, 13.7 ms before, 11.8 now):
+// run through the same phases together. Some 4,300 cycles per tile before the changes below; clock stamps with the
+// first two of them in place: 2,500 in the scale loop, 680 for the row maxima, 740 for exp and P, 310 - 360 for barriers
+// that had long completed. What was changed (2,048 tokens behind 148,000, 13.7 ms before, 11.8 now):
 //  * The accumulators are read in the fragment layout of a warp MMA (tcgen05.ld.16x256b): a thread holds 4 rows x 8
 //    positions instead of 1 x 32, and loads 8 K scales and 4 Q scales per block instead of 32 and 1. A 16-byte
 //    shared-memory load returns 512 bytes to the warp whether its threads read one address or 32.
