@@ -63,7 +63,7 @@ constexpr int P_WORDS = MAXR * P_STRIDE;
 constexpr int Q_STRIDE = 2 * AD + 16;             // bytes per staged Q row (f16; 16 bytes of padding: conflict-free 16-byte reads)
 constexpr int SCHED_DONE = 32;                    // p.sched: [KV head] pool counters, [32] CTAs that are done
 constexpr float TAU = 8.0f;                       // a score may exceed the reference max by this much
-constexpr int O_STRIDE = AD + 4;                  // floats per row of the end-of-kernel O exchange
+constexpr int O_XCH_BYTES = 128 * 12 * 16;        // end-of-kernel O exchange: [12][128 threads] float4, the accumulators of half a thread
 
 // Shared memory map of a CTA with NG tile groups (offsets from a 1024-byte aligned base). NG = 2: the
 // default, one CTA of 16 warps per SM. NG = 1: 8 warps and half the rings, two CTAs per SM, for launches of
@@ -83,13 +83,15 @@ struct Lay {
   static constexpr int OFF_M1 = OFF_L + NG * 4 * MAXR * 4;           // [NG groups][24] floats: reference maxima at the end
   static constexpr int OFF_BAR = OFF_M1 + NG * MAXR * 4;             // fullK[NG * KDEPTH], fullV[NG * VDEPTH]
   static constexpr int OFF_FLAG = OFF_BAR + NG * (KDEPTH + VDEPTH) * 8;
+  static constexpr int OFF_GROUP1 = OFF_FLAG + 4;                    // tiles that group 1 had (its Q K^T warps, at their end)
   static constexpr int OFF_TOK = OFF_FLAG + 16;                      // [2 groups][2 buffers] words: "move the maxima" tokens (QK warps)
   static constexpr int OFF_RTOK = OFF_TOK + 16;                      // [2 groups][2 buffers] words: "rescale O" tokens (QK -> PV)
   static constexpr int OFF_SEQ = OFF_RTOK + 16;                      // [2 groups][8] ints: the groups' tile queues
   static constexpr int SMEM_USED = OFF_SEQ + 64;
   static constexpr int SMEM_BYTES = SMEM_USED + 1024;                // slack for the 1024-byte alignment of the ring
   static_assert(OFF_BAR % 8 == 0, "mbarriers are 8-byte aligned");
-  static_assert(NG == 1 || MAXR * O_STRIDE * 4 <= RING_BYTES, "O exchange must fit in the ring");
+  static constexpr int OFF_STAGE = NG == 2 ? O_XCH_BYTES : 0;        // the chunk partial before it is written out, over the ring as well
+  static_assert(OFF_STAGE + MAXR * PROW * 4 <= RING_BYTES, "O exchange and partial must fit in the ring");
   static_assert(SMEM_BYTES * (3 - NG) + (3 - NG) * 1024 <= 232448, "shared memory of one SM");
 };
 
@@ -103,6 +105,7 @@ constexpr int BAR_QK = 1;      // + group: the four QK warps of a group
 constexpr int BAR_READY = 3;   // + 2 * group + buffer: P tile written (QK arrives, PV waits)
 constexpr int BAR_FREE = 7;    // + 2 * group + buffer: P tile consumed (PV arrives, QK waits)
 constexpr int BAR_QKALL = 11;  // all QK warps of the CTA, once, at their end
+constexpr int BAR_PVALL = 12;  // all PV warps of the CTA, once, when the partial is staged
 
 __device__ __forceinline__ uint32_t lds32(uint32_t a) {
   uint32_t v;
@@ -129,6 +132,9 @@ __device__ __forceinline__ void sts64(uint32_t a, uint32_t x, uint32_t y) {
   asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(a), "r"(x), "r"(y) : "memory");
 }
 __device__ __forceinline__ void stsf(uint32_t a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
+__device__ __forceinline__ void sts128f(uint32_t a, const float (&v)[4]) {
+  asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(a), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+}
 __device__ __forceinline__ float ldsf(uint32_t a) {
   float v;
   asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
@@ -378,7 +384,8 @@ decode_ws_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constan
 #define PROF_BEGIN()
 #define PROF_END(acc)
 #endif
-    for (int jt = 0;; jt++) {
+    int jt = 0;
+    for (;; jt++) {
       const int tile = (int)lds32(sSeq + (jt & 7) * 4);
       if (tile < 0) break;
       const int s = NG * (jt % KDEPTH) + grp;
@@ -561,6 +568,7 @@ decode_ws_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constan
     // of the grid to say so puts the counters back to zero for the next launch. This is done now, while the
     // P V warps are still a tile behind: the fence and the atomic take more than a microsecond, and between
     // the CTA's two barriers below the P V warps would wait for them.
+    if (NG == 2 && tid == 128) sts32(sbase + L::OFF_GROUP1, (uint32_t)jt);
     if (NG == 2) bar_sync(BAR_QKALL, 256);
     if (has_pool && tid == 0) {
       __threadfence();
@@ -572,7 +580,7 @@ decode_ws_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constan
       }
     }
     __syncthreads();  // every tile consumed: the ring is free for the O exchange
-    if (NG == 2) __syncthreads();  // (the P V warps' barrier between the two halves of their exchange)
+    if (NG == 2 && lds32(sbase + L::OFF_GROUP1) != 0) __syncthreads();  // (the P V warps' barrier between the two halves of their exchange)
     return;
   }
 
@@ -707,50 +715,54 @@ decode_ws_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constan
 #endif
   __syncthreads();  // every tile consumed: the ring is free for the O exchange; m and l are posted
 
-  if constexpr (NG == 1) {  // one group: its accumulators, maxima and sums are the chunk partial
+  // The partial is put together in shared memory as it is in global memory ([row][m, l, O]) and then copied out 16
+  // bytes a thread, in order, by all P V warps: written straight from the accumulators of one group it is 48 8-byte
+  // stores a thread that touch 32 sectors each. The groups are merged thread to thread; a chunk of a single tile
+  // (group 1 had none) skips that. Layer behind 1,024 positions 11.4 -> 11.1 us, behind 32,768 26.8 -> 26.4, 150,000
+  // 75.0 -> 74.1. (The same in decode.cu, whose eight warps all hold accumulators, was 2 % slower and is not done there.)
+  const uint32_t sStage = sbase + L::OFF_STAGE;
+  if (NG == 1 || lds32(sbase + L::OFF_GROUP1) == 0) {  // one group: its accumulators, maxima and sums are the chunk partial
 #pragma unroll
     for (int nt = 0; nt < NT; nt++)
 #pragma unroll
       for (int e = 0; e < 2; e++) {
         const int r = 8 * nt + 2 * tg + e;
-        if (r >= R) continue;
-        float* po = out + (size_t)r * PROW;
+        if (r >= R || grp != 0) continue;
+        const uint32_t row = sStage + r * (PROW * 4);
 #pragma unroll
-        for (int mt = 0; mt < 4; mt++) {
-          const int d = 64 * wq + 8 * g + 2 * mt;
-          *(float2*)(po + 2 + d) = make_float2(o[mt][nt][e], o[mt][nt][2 + e]);
-        }
+        for (int mt = 0; mt < 4; mt++)
+          sts64(row + 8 + (64 * wq + 8 * g + 2 * mt) * 4, __float_as_uint(o[mt][nt][e]), __float_as_uint(o[mt][nt][2 + e]));
         if (wq == 0 && g == 0) {
           float l0 = 0.f;
 #pragma unroll
           for (int w = 0; w < 4; w++) l0 += ldsf(sbase + OFF_L + (w * MAXR + r) * 4);
-          po[0] = ldsf(sbase + OFF_M1 + r * 4);
-          po[1] = l0;
+          sts64(row, __float_as_uint(ldsf(sbase + OFF_M1 + r * 4)), __float_as_uint(l0));
         }
       }
-    if (tid == PV0) stamp(7);
-    return;
-  }
-  // ---- merge the two groups (log-sum-exp) and write the chunk partial
-  const uint32_t sO = sbase;
-  if (grp == 1) {
+  } else if constexpr (NG == 2) {
+    // Merge the two groups (log-sum-exp). Thread i of either group holds the same rows and dims, so the accumulators
+    // travel thread to thread, 16 bytes side by side: group 1 hands over the lower half of its dims and group 0 the
+    // upper half, and each group merges the half it kept.
+    const uint32_t sX = sbase + wq * 512 + lane * 16;  // float4 c of this thread (2 dims x 2 rows) at sX + 2048 c
 #pragma unroll
     for (int nt = 0; nt < NT; nt++)
 #pragma unroll
-      for (int e = 0; e < 2; e++) {
-        const int r = 8 * nt + 2 * tg + e;
+      for (int u = 0; u < 2; u++) {
+        float x[4];
 #pragma unroll
-        for (int mt = 0; mt < 4; mt++) {
-          const int d = 64 * wq + 8 * g + 2 * mt;
-          stsf(sO + (r * O_STRIDE + d) * 4, o[mt][nt][e]);
-          stsf(sO + (r * O_STRIDE + d + 1) * 4, o[mt][nt][2 + e]);
-        }
+        for (int i = 0; i < 4; i++) x[i] = grp == 0 ? o[2 + u][nt][i] : o[u][nt][i];
+        sts128f(sX + (grp * 6 + 2 * nt + u) * 2048, x);
       }
-  }
-  __syncthreads();
-  if (grp == 0) {
+    __syncthreads();
 #pragma unroll
-    for (int nt = 0; nt < NT; nt++)
+    for (int nt = 0; nt < NT; nt++) {
+      float x[2][4];
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const uint4 w = lds128(sX + ((grp ^ 1) * 6 + 2 * nt + u) * 2048);
+        x[u][0] = __uint_as_float(w.x); x[u][1] = __uint_as_float(w.y);
+        x[u][2] = __uint_as_float(w.z); x[u][3] = __uint_as_float(w.w);
+      }
 #pragma unroll
       for (int e = 0; e < 2; e++) {
         const int r = 8 * nt + 2 * tg + e;
@@ -758,27 +770,29 @@ decode_ws_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constan
         const float m0 = ldsf(sbase + OFF_M1 + r * 4), m1 = ldsf(sbase + OFF_M1 + (MAXR + r) * 4);
         const float M = fmaxf(m0, m1);
         const float f0 = ex2((m0 - M) * LOG2E), f1 = ex2((m1 - M) * LOG2E);
-        float* po = out + (size_t)r * PROW;
+        const uint32_t row = sStage + r * (PROW * 4);
 #pragma unroll
-        for (int mt = 0; mt < 4; mt++) {
-          const int d = 64 * wq + 8 * g + 2 * mt;
-          const float v0 = o[mt][nt][e] * f0 + ldsf(sO + (r * O_STRIDE + d) * 4) * f1;
-          const float v1 = o[mt][nt][2 + e] * f0 + ldsf(sO + (r * O_STRIDE + d + 1) * 4) * f1;
-          *(float2*)(po + 2 + d) = make_float2(v0, v1);
+        for (int u = 0; u < 2; u++) {
+          const float a0 = grp == 0 ? o[u][nt][e] : o[2 + u][nt][e], a1 = grp == 0 ? o[u][nt][2 + e] : o[2 + u][nt][2 + e];
+          const float v0 = grp == 0 ? a0 * f0 + x[u][e] * f1 : x[u][e] * f0 + a0 * f1;
+          const float v1 = grp == 0 ? a1 * f0 + x[u][2 + e] * f1 : x[u][2 + e] * f0 + a1 * f1;
+          sts64(row + 8 + (64 * wq + 8 * g + 2 * (2 * grp + u)) * 4, __float_as_uint(v0), __float_as_uint(v1));
         }
-        if (wq == 0 && g == 0) {
+        if (grp == 0 && wq == 0 && g == 0) {
           float l0 = 0.f, l1 = 0.f;
 #pragma unroll
           for (int w = 0; w < 4; w++) {
             l0 += ldsf(sbase + OFF_L + (w * MAXR + r) * 4);
             l1 += ldsf(sbase + OFF_L + ((4 + w) * MAXR + r) * 4);
           }
-          po[0] = M;
-          po[1] = l0 * f0 + l1 * f1;
+          sts64(row, __float_as_uint(M), __float_as_uint(l0 * f0 + l1 * f1));
         }
       }
-    if (tid == PV0) stamp(7);
+    }
   }
+  bar_sync(BAR_PVALL, 128 * NG);
+  for (int i = tid - PV0; i < R * PROW / 4; i += 128 * NG) ((uint4*)out)[i] = lds128(sStage + 16 * i);  // R is a multiple of 6
+  if (tid == PV0) stamp(7);
 }
 
 template <int NT, int NG>
