@@ -14,20 +14,19 @@
 namespace {
 
 enum Fn { PREP, DECODE, PREP_PAGED, DECODE_PAGED, PREFILL, N_FN };
-void* g_fn[N_FN];
-PyObject* g_ptr = nullptr;    // _ptr(tensor, dtype, optional) -> ctypes.c_void_p
-PyObject* g_check = nullptr;  // _check(return code): raises
-PyObject* g_f32 = nullptr;    // torch.float32, int32, int8 as Python objects, for g_ptr
-PyObject* g_i32 = nullptr;
-PyObject* g_i8 = nullptr;
-
-
-PyObject* dtype_object(c10::ScalarType t) {
-  return t == c10::kFloat ? g_f32 : t == c10::kInt ? g_i32 : t == c10::kChar ? g_i8 : Py_None;
+// One per module object: the package may be loaded under two names, each with its own library and error class.
+struct State {
+  void* fn[N_FN];
+  PyObject* ptr;    // _ptr(tensor, dtype, optional) -> ctypes.c_void_p
+  PyObject* check;  // _check(return code): raises
+  PyObject *f32, *i32, *i8;  // torch.float32, int32, int8 as Python objects, for ptr
+};
+PyObject* dtype_object(const State* st, c10::ScalarType t) {
+  return t == c10::kFloat ? st->f32 : t == c10::kInt ? st->i32 : t == c10::kChar ? st->i8 : Py_None;
 }
 
 // Device address of one tensor argument. want = Undefined: any dtype.
-bool ptr(PyObject* o, c10::ScalarType want, bool optional, void** out) {
+bool ptr(const State* st, PyObject* o, c10::ScalarType want, bool optional, void** out) {
   if (THPVariable_CheckExact(o)) {
     const at::Tensor& t = THPVariable_Unpack(o);
     if (t.is_cuda() && t.is_contiguous() && (want == c10::ScalarType::Undefined || t.scalar_type() == want)) {
@@ -35,7 +34,7 @@ bool ptr(PyObject* o, c10::ScalarType want, bool optional, void** out) {
       return true;
     }
   }
-  PyObject* r = PyObject_CallFunctionObjArgs(g_ptr, o, dtype_object(want), optional ? Py_True : Py_False, nullptr);
+  PyObject* r = PyObject_CallFunctionObjArgs(st->ptr, o, dtype_object(st, want), optional ? Py_True : Py_False, nullptr);
   if (!r) return false;
   PyObject* v = PyObject_GetAttrString(r, "value");
   Py_DECREF(r);
@@ -65,19 +64,21 @@ bool flag(PyObject* o, int* out) {
   return t >= 0;
 }
 
-PyObject* done(int rc) {
+PyObject* done(const State* st, int rc) {
   if (rc == 0) Py_RETURN_NONE;
-  return PyObject_CallFunction(g_check, "i", rc);
+  return PyObject_CallFunction(st->check, "i", rc);
 }
 
 constexpr c10::ScalarType F32 = c10::kFloat, I32 = c10::kInt, I8 = c10::kChar, ANY = c10::ScalarType::Undefined;
 
 // Runs `body`, turning C++ exceptions of torch into Python errors.
 template <class B>
-PyObject* guarded(Py_ssize_t n, Py_ssize_t want, B body) {
+PyObject* guarded(PyObject* self, Py_ssize_t n, Py_ssize_t want, B body) {
+  const State* st = (const State*)PyModule_GetState(self);
+  if (!st || !st->ptr) return PyErr_Format(PyExc_RuntimeError, "q27b_binding is not bound");
   if (n != want) return PyErr_Format(PyExc_TypeError, "expected %zd arguments, got %zd", want, n);
   try {
-    return body();
+    return body(st);
   } catch (const std::exception& e) {
     if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, e.what());
     return nullptr;
@@ -87,7 +88,7 @@ void* stream() { return (void*)c10::cuda::getCurrentCUDAStream().stream(); }
 
 #define PTR(i, type, opt, name) \
   void* name;                   \
-  if (!ptr(a[i], type, opt, &name)) return nullptr
+  if (!ptr(st, a[i], type, opt, &name)) return nullptr
 #define NUM(i, name) \
   int name;          \
   if (!num(a[i], &name)) return nullptr
@@ -97,17 +98,17 @@ void* stream() { return (void*)c10::cuda::getCurrentCUDAStream().stream(); }
 #define FLAG(i, name) \
   int name;           \
   if (!flag(a[i], &name)) return nullptr
-#define CALL(fn, type, ...)          \
+#define CALL(which, type, ...)             \
   void* s = stream();                \
   int rc;                            \
   Py_BEGIN_ALLOW_THREADS             \
-  rc = ((type)g_fn[fn])(__VA_ARGS__); \
+  rc = ((type)st->fn[which])(__VA_ARGS__); \
   Py_END_ALLOW_THREADS               \
-  return done(rc)
+  return done(st, rc)
 
 // qg, k, v, q_norm, k_norm, qn, kcache, vcache, pos0, T, eps, theta_scale, nqh, nkvh, n_ctx, q8, rope3, rdelta
-PyObject* attn_prep(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  return guarded(n, 18, [&]() -> PyObject* {
+PyObject* attn_prep(PyObject* self, PyObject* const* a, Py_ssize_t n) {
+  return guarded(self, n, 18, [&](const State* st) -> PyObject* {
     PTR(0, F32, false, qg); PTR(1, F32, false, k); PTR(2, F32, false, v); PTR(3, F32, false, qw); PTR(4, F32, false, kw);
     PTR(5, F32, false, qn); PTR(6, ANY, false, kc); PTR(7, ANY, false, vc); PTR(8, I32, false, pos0);
     NUM(9, T); FLT(10, eps); FLT(11, theta); NUM(12, nqh); NUM(13, nkvh); NUM(14, n_ctx); FLAG(15, q8);
@@ -118,8 +119,8 @@ PyObject* attn_prep(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // qn, qg, kcache, vcache, o, xq, xd, pos0, T, kq_scale, nqh, nkvh, n_ctx, q8
-PyObject* attn_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  return guarded(n, 14, [&]() -> PyObject* {
+PyObject* attn_decode(PyObject* self, PyObject* const* a, Py_ssize_t n) {
+  return guarded(self, n, 14, [&](const State* st) -> PyObject* {
     PTR(0, F32, false, qn); PTR(1, F32, false, qg); PTR(2, ANY, false, kc); PTR(3, ANY, false, vc); PTR(4, F32, true, o);
     PTR(5, I8, true, xq); PTR(6, F32, true, xd); PTR(7, I32, false, pos0);
     NUM(8, T); FLT(9, scale); NUM(10, nqh); NUM(11, nkvh); NUM(12, n_ctx); FLAG(13, q8);
@@ -129,8 +130,8 @@ PyObject* attn_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // qg, k, v, q_norm, k_norm, qn, kpool, vpool, page_table, seq_len, B, T, eps, theta_scale, nqh, nkvh, n_pages, max_pages, rope3, rdelta
-PyObject* attn_prep_paged(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  return guarded(n, 20, [&]() -> PyObject* {
+PyObject* attn_prep_paged(PyObject* self, PyObject* const* a, Py_ssize_t n) {
+  return guarded(self, n, 20, [&](const State* st) -> PyObject* {
     PTR(0, F32, true, qg); PTR(1, F32, false, k); PTR(2, F32, false, v); PTR(3, F32, true, qw); PTR(4, F32, true, kw);
     PTR(5, F32, true, qn); PTR(6, ANY, false, kp); PTR(7, ANY, false, vp); PTR(8, I32, false, table); PTR(9, I32, false, lens);
     NUM(10, B); NUM(11, T); FLT(12, eps); FLT(13, theta); NUM(14, nqh); NUM(15, nkvh); NUM(16, n_pages); NUM(17, max_pages);
@@ -141,8 +142,8 @@ PyObject* attn_prep_paged(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // qn, qg, kpool, vpool, page_table, seq_len, o, B, T, kq_scale, nqh, nkvh, n_pages, max_pages, max_seq_len
-PyObject* attn_decode_paged(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  return guarded(n, 15, [&]() -> PyObject* {
+PyObject* attn_decode_paged(PyObject* self, PyObject* const* a, Py_ssize_t n) {
+  return guarded(self, n, 15, [&](const State* st) -> PyObject* {
     PTR(0, F32, false, qn); PTR(1, F32, false, qg); PTR(2, ANY, false, kp); PTR(3, ANY, false, vp); PTR(4, I32, false, table);
     PTR(5, I32, false, lens); PTR(6, F32, false, o);
     NUM(7, B); NUM(8, T); FLT(9, scale); NUM(10, nqh); NUM(11, nkvh); NUM(12, n_pages); NUM(13, max_pages); NUM(14, max_len);
@@ -152,8 +153,8 @@ PyObject* attn_decode_paged(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // qn, qg, kcache, vcache, o, pos0, M, kq_scale, nqh, nkvh, n_ctx, q8, depth_hint
-PyObject* attn_prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  return guarded(n, 13, [&]() -> PyObject* {
+PyObject* attn_prefill(PyObject* self, PyObject* const* a, Py_ssize_t n) {
+  return guarded(self, n, 13, [&](const State* st) -> PyObject* {
     PTR(0, F32, false, qn); PTR(1, F32, false, qg); PTR(2, ANY, false, kc); PTR(3, ANY, false, vc); PTR(4, F32, false, o);
     PTR(5, I32, false, pos0);
     NUM(6, M); FLT(7, scale); NUM(8, nqh); NUM(9, nkvh); NUM(10, n_ctx); FLAG(11, q8); NUM(12, depth);
@@ -163,22 +164,24 @@ PyObject* attn_prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // addresses (tuple of N_FN ints), _ptr, _check, torch.float32, torch.int32, torch.int8
-PyObject* bind(PyObject*, PyObject* args) {
+PyObject* bind(PyObject* self, PyObject* args) {
   PyObject *fns, *p, *c, *f32, *i32, *i8;
   if (!PyArg_ParseTuple(args, "O!OOOOO", &PyTuple_Type, &fns, &p, &c, &f32, &i32, &i8)) return nullptr;
   if (PyTuple_GET_SIZE(fns) != N_FN) return PyErr_Format(PyExc_ValueError, "expected %d addresses", (int)N_FN);
-  for (int i = 0; i < N_FN; i++) g_fn[i] = PyLong_AsVoidPtr(PyTuple_GET_ITEM(fns, i));
+  State* st = (State*)PyModule_GetState(self);
+  for (int i = 0; i < N_FN; i++) st->fn[i] = PyLong_AsVoidPtr(PyTuple_GET_ITEM(fns, i));
   if (PyErr_Occurred()) return nullptr;
-  Py_XSETREF(g_ptr, Py_NewRef(p)); Py_XSETREF(g_check, Py_NewRef(c));
-  Py_XSETREF(g_f32, Py_NewRef(f32)); Py_XSETREF(g_i32, Py_NewRef(i32)); Py_XSETREF(g_i8, Py_NewRef(i8));
+  Py_XSETREF(st->ptr, Py_NewRef(p)); Py_XSETREF(st->check, Py_NewRef(c));
+  Py_XSETREF(st->f32, Py_NewRef(f32)); Py_XSETREF(st->i32, Py_NewRef(i32)); Py_XSETREF(st->i8, Py_NewRef(i8));
   Py_RETURN_NONE;
 }
 
 #define FAST(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
 PyMethodDef g_methods[] = {{"bind", bind, METH_VARARGS, nullptr}, FAST(attn_prep), FAST(attn_decode), FAST(attn_prep_paged),
                            FAST(attn_decode_paged), FAST(attn_prefill), {nullptr, nullptr, 0, nullptr}};
-PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "q27b_binding", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};
+PyModuleDef_Slot g_slots[] = {{0, nullptr}};
+PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "q27b_binding", nullptr, sizeof(State), g_methods, g_slots, nullptr, nullptr, nullptr};
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit_q27b_binding(void) { return PyModule_Create(&g_module); }
+PyMODINIT_FUNC PyInit_q27b_binding(void) { return PyModuleDef_Init(&g_module); }

@@ -264,3 +264,18 @@ def test_native_binding_checks_like_the_python_layer(q27):
         q27.attn_decode(*args[:-1])
     with pytest.raises(AttributeError):
         q27.attn_prefill("not a tensor", *args[1:5], 0, 4, 0.1, 24, 4, 100)
+
+
+def test_binding_state_belongs_to_the_package_object(q27):
+    """The package loaded a second time under another name has its own error class (and may have its own library): the
+    first one keeps its own."""
+    import importlib.util
+    path = os.path.join(os.path.dirname(q27.__file__), "__init__.py")
+    spec = importlib.util.spec_from_file_location("q27_second_load", path, submodule_search_locations=[os.path.dirname(path)])
+    other = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(other)
+    t = torch.zeros(4)
+    for m, n in ((q27, other), (other, q27)):
+        with pytest.raises(m.Q27Error) as e:
+            m.attn_decode(t, 0, 0, 0, 0, None, None, 0, 4, 0.1, 24, 4, 100)
+        assert not isinstance(e.value, n.Q27Error)
