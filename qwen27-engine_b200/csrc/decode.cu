@@ -283,6 +283,16 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constant__
   const uint32_t vC = vQ + (vrow + 1) * 128 + ((vcb ^ ((vrow + 1) & 7)) << 4);
   const uint32_t sA = G::OFF_VS + (2 * wq + (g >> 2)) * 2 + vrow * 16;
 
+  if (NSTAGE % NGROUP != 0 && ntiles > NSTAGE) {
+    // With an odd number of stages a stage passes from one group to the other. A group must not come to wait for the
+    // second tile of a stage while the first one, the other group's, has not landed: the parity of that wait is then
+    // already the barrier's. Later tiles are safe, since each is requested by the other group from inside its tile; the
+    // first ones are requested at once. So nobody starts before tiles 0 and 1 are there (nothing is requested before
+    // either, and a barrier that had moved on twice could not be asked).
+    mbar_wait(&full[0], 0, abort_flag, p.status);
+    mbar_wait(&full[1], 0, abort_flag, p.status);
+    bar_sync(BAR_ALL, N_THREADS);
+  }
   int jt = 0;
   for (int it = grp; it < ntiles; it += NGROUP, jt++) {
     const int s = it % NSTAGE;

@@ -365,3 +365,22 @@ def test_step_captured_behind_a_copy_and_another_stream(q27, orc):
         assert_close(got.cpu().numpy(), o2.cpu().numpy(), "replay at n=%d" % n)
         assert torch.equal(kc, kc2) and torch.equal(vc, vc2)
     assert q27.device_status() == 0
+
+
+@pytest.mark.parametrize("T", [1, 2])
+def test_f16_cache_many_tiles_a_chunk(q27, orc, T):
+    """Few query tokens over 13 tiles a chunk of an f16 cache: the two tile groups share an odd number of stages, and a
+    fast group must not take the other's first tile for its own next one."""
+    from qwen27_engine_b200 import synth
+    nkvh, n = 1, 120007
+    nqh, n_ctx = nkvh * GQA, n + 9
+    qn, qg, kf, vf = synth.decode_inputs(T, nqh, nkvh, n)
+    kc_ref, vc_ref = orc.fill_cache(kf, vf, n_ctx, q8=False)
+    kc, vc = poisoned_cache(q27, kc_ref, nkvh, n_ctx, n, False), poisoned_cache(q27, vc_ref, nkvh, n_ctx, n, False)
+    ref = orc.attn_ref(qn, qg, kc_ref, vc_ref, n - T, SCALE, nkvh, n_ctx, q8=False)
+    for _ in range(5):
+        o = torch.full((T, nqh, AD), float("nan"), device="cuda")
+        q27.attn_decode(dev(qn), dev(qg), kc, vc, o, None, None, pos_tensor(n - T), T, SCALE, nqh, nkvh, n_ctx, False)
+        torch.cuda.synchronize()
+        assert_close(o.cpu().numpy(), ref, "f16 T=%d n=%d" % (T, n))
+    assert q27.device_status() == 0
