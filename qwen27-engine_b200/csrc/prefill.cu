@@ -39,7 +39,9 @@
 //  * No int -> float conversion: an MMA of constants (-128 * -128 * 32 = 2^19, for two slots at once) puts an offset
 //    under the block sums, so that they are positive and below 2^20; read as bits of a float, such an integer n is the
 //    subnormal n * 2^-149, and one FMA with the K scale (times 2^110) takes the offset off again and rounds once:
-//    dk * I as exactly as the converted form. The powers of two cancel against the Q scale (times 2^39).
+//    dk * I as exactly as the converted form. The scores of the loop are therefore in units of 2^39, which the constants
+//    of the softmax take out: the Q scale itself stays as it is, so that no finite one overflows. An infinite K scale
+//    makes inf - inf of every sum of its block, and NaN of every row that sees the position.
 //  * A vote of the two warps of a row quarter (bar.red) replaces the exchange of row maxima; maxima are exchanged only
 //    when one moves.
 //  * The scale table has a barrier of its own and is ready long before V; the softmax warps wait for neither: the
@@ -148,9 +150,11 @@ struct PrefillParams {
   float* xd;       // ... and one scale per 32 values, as f32(f16(d)) (q8_store, src/common.cuh:72-81)
 };
 
-// Powers of two that bring subnormal block sums (n * 2^-149) into the range of normal numbers; 2^(110 + 39) takes them out
-// again. An f16 scale times 2^110 stays below 2^126, a product with a block sum above 2^-63.
-constexpr float DK_SCALE = 0x1p110f, DQ_SCALE = 0x1p39f, OFS_SCALE = -0x1p-130f;  // OFS_SCALE: -2^19 * 2^-149
+// The K scales carry 2^110, which brings subnormal block sums (n * 2^-149) into the range of normal numbers: an f16 scale
+// times 2^110 stays below 2^126, a product with a block sum above 2^-63. Scores and reference maxima are held in units of
+// 2^39; every constant that meets one carries the power of two, so that all roundings are those of the plain form.
+constexpr float DK_SCALE = 0x1p110f, OFS_SCALE = -0x1p-130f;  // OFS_SCALE: -2^19 * 2^-149
+constexpr float S_UNIT = 0x1p39f, M_INIT_S = M_INIT / S_UNIT, TAU_S = TAU / S_UNIT, LOG2E_S = LOG2E * S_UNIT;
 
 // Barrier of the NWG threads' warps that share query rows 32q .. 32q+31.
 __device__ __forceinline__ void pair_sync(int q) { asm volatile("bar.sync %0, %1;" ::"r"(1 + q), "n"(32 * NWG) : "memory"); }
@@ -339,7 +343,7 @@ prefill_i8_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_consta
       else quantise_q_row<NB, NB>(src, p.kq_scale, sgen + OFF_Q, r, dqh);
 #pragma unroll
       for (int i = 0; i < NB; i++)
-        *(float*)(sgen + OFF_DQ + (((NB * wg + i) * 4 + q) * 8 + (lane & 7)) * 16 + (lane >> 3) * 4) = dqh[i] * DQ_SCALE;
+        *(float*)(sgen + OFF_DQ + (((NB * wg + i) * 4 + q) * 8 + (lane & 7)) * 16 + (lane >> 3) * 4) = dqh[i];
       if (wg == 0) {
         const uint4 w = make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u);
         *(uint4*)(sgen + OFF_OFS + r * 32) = w;
@@ -360,10 +364,10 @@ prefill_i8_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_consta
     uint64_t l2[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      m_ref[k] = M_INIT;
+      m_ref[k] = M_INIT_S;
       l2[k] = pack2(0.f, 0.f);
     }
-    const uint64_t log2e2 = pack2(LOG2E, LOG2E);
+    const uint64_t log2e2 = pack2(LOG2E_S, LOG2E_S);
     const uint64_t ofs2 = pack2(OFS_SCALE, OFS_SCALE);
 
 #pragma unroll 1
@@ -436,7 +440,7 @@ prefill_i8_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_consta
 #pragma unroll
       for (int k = 0; k < 4; k++) {
         mt[k] = fmaxf(fmaxf(fmaxf(s[k][0], s[k][1]), fmaxf(s[k][2], s[k][3])), fmaxf(fmaxf(s[k][4], s[k][5]), fmaxf(s[k][6], s[k][7])));
-        want |= mt[k] > m_ref[k] + TAU;
+        want |= mt[k] > m_ref[k] + TAU_S;
       }
       if (pair_any(q, want)) {
         float f[4];
@@ -453,7 +457,7 @@ prefill_i8_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_consta
 #pragma unroll
         for (int k = 0; k < 4; k++) {
           const float m = fmaxf(m_ref[k], fmaxf(mt[k], ot[k]));
-          f[k] = ex2((m_ref[k] - m) * LOG2E);  // 0 on the first move (m_ref = -1e30)
+          f[k] = ex2((m_ref[k] - m) * LOG2E_S);  // 0 on the first move (m_ref = -1e30)
           m_ref[k] = m;
           l2[k] = mul2(l2[k], pack2(f[k], f[k]));
         }
@@ -472,7 +476,7 @@ prefill_i8_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_consta
       uint8_t* sP = sgen + OFF_P + pb * P_BYTES + (q * 32 + g) * 128 + 4 * tg;
 #pragma unroll
       for (int k = 0; k < 4; k++) {
-        const float nmb = -m_ref[k] * LOG2E;
+        const float nmb = -m_ref[k] * LOG2E_S;
         const uint64_t nmb2 = pack2(nmb, nmb);
 #pragma unroll
         for (int i = 0; i < 4; i++) {
@@ -505,7 +509,7 @@ prefill_i8_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_consta
       const float4 o4 = *(const float4*)(xch + (wg ^ 1) * QT);
       l4[0] += o4.x; l4[1] += o4.y; l4[2] += o4.z; l4[3] += o4.w;
     }
-    const float l = row_of_lane(l4, lane), m_row = row_of_lane(m_ref, lane);
+    const float l = row_of_lane(l4, lane), m_row = row_of_lane(m_ref, lane) * S_UNIT;
     pf_wait(&bar[B_ODONE], 0, abort_flag, p.status);
     tc_fence_after();
     const float inv_l = 1.0f / l;
@@ -608,12 +612,10 @@ prefill_i8_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_consta
           const uint2 sc = *(const uint2*)(kst + 2 * PT * 128 + row * 16 + b0 * 2);
           const __half2 s01 = u32_as_h2(sc.x), s23 = u32_as_h2(sc.y);
           const float d4[4] = {__low2float(s01), __high2float(s01), __low2float(s23), __high2float(s23)};
-          // An infinite scale (a K value above 8.3 million) counts as the largest finite one: the offset of the block sums
-          // must cancel, inf - inf would not.
           // position row = 32 wg + 8 i + 2 tg + e -> [block][wg][tg][i][e]
           float* dst = dkf + (row >> 5) * 32 + ((row >> 1) & 3) * 8 + ((row >> 3) & 3) * 2 + (row & 1);
 #pragma unroll
-          for (int i = 0; i < 4; i++) dst[(b0 + i) * PT] = (d4[i] == INFINITY ? 65504.f : d4[i]) * DK_SCALE;
+          for (int i = 0; i < 4; i++) dst[(b0 + i) * PT] = d4[i] * DK_SCALE;
         }
       }
       __syncwarp();

@@ -380,3 +380,51 @@ def test_prefill_i8_magnitudes(q27, orc, qs, ks):
     # size of V itself, so the bound is relative to their RMS
     assert_close(o.cpu().numpy(), ref, "qs=%g ks=%g" % (qs, ks), abs_tol=1e-2 * float(np.sqrt((ref.astype(np.float64) ** 2).mean())))
     assert q27.device_status() == 0
+
+
+@pytest.mark.parametrize("qs", [1e28, 1e30, 1e36])
+@pytest.mark.parametrize("depth_hint", [-1, 333])
+def test_prefill_i8_large_q(q27, orc, qs, depth_hint):
+    """Q scales from 2^82, 2^89 and 2^108 on in two blocks whose K values are zero: the scores are those of the other blocks.
+    (Large scores themselves are no test: beyond some 1e9 the rounding of score times log2(e) decides the exponent.)"""
+    from qwen27_engine_b200 import synth
+    pos0, M, nkvh = 333, 60, 1
+    nqh, n = nkvh * GQA, pos0 + M
+    n_ctx = n + 9
+    qn, qg, _, vc_ref, n, n_ctx = make_case(orc, M, pos0, nkvh, n_ctx)
+    kf = synth.normal(synth.SEED_K, (nkvh, n, AD)).copy()
+    for b in (0, 5):
+        qn[..., 32 * b:32 * b + 32] *= np.float32(qs)
+        kf[..., 32 * b:32 * b + 32] = 0
+    kc_ref, _ = orc.fill_cache(kf, kf, n_ctx)
+    ref = orc.attn_prefill_i8(qn, qg, kc_ref, vc_ref, pos0, SCALE, nkvh, n_ctx)
+    o = torch.full((M, nqh, AD), float("nan"), device="cuda")
+    q27.attn_prefill(dev(qn), dev(qg), dev(kc_ref), dev(vc_ref), o, pos_tensor(pos0), M, SCALE, nqh, nkvh, n_ctx,
+                     depth_hint=depth_hint)
+    torch.cuda.synchronize()
+    assert_close(o.cpu().numpy(), ref, "qs=%g" % qs)
+    assert q27.device_status() == 0
+
+
+@pytest.mark.parametrize("depth_hint", [-1, 333])
+def test_prefill_i8_infinite_k_scale_stays_visible(q27, orc, depth_hint):
+    """A K row whose f16 scale overflowed: every row that sees it is NaN, as decode over the same cache is; rows before it
+    are untouched."""
+    from qwen27_engine_b200 import synth
+    pos0, M, nkvh, first = 333, 60, 1, 27
+    nqh, n = nkvh * GQA, pos0 + M
+    n_ctx = n + 9
+    qn, qg, kc_ref, vc_ref, n, n_ctx = make_case(orc, M, pos0, nkvh, n_ctx)
+    ref = orc.attn_prefill_i8(qn, qg, kc_ref, vc_ref, pos0, SCALE, nkvh, n_ctx)
+    kc = np.array(kc_ref, copy=True)
+    kc[nkvh * n_ctx * AD:].view(np.float16).reshape(nkvh, n_ctx, 8)[0, pos0 + first, 3] = np.inf
+    o = torch.full((M, nqh, AD), 7.0, device="cuda")
+    q27.attn_prefill(dev(qn), dev(qg), dev(kc), dev(vc_ref), o, pos_tensor(pos0), M, SCALE, nqh, nkvh, n_ctx,
+                     depth_hint=depth_hint)
+    o4 = torch.full((4, nqh, AD), 7.0, device="cuda")
+    q27.attn_decode(dev(qn[-4:]), dev(qg[-4:]), dev(kc), dev(vc_ref), o4, None, None, pos_tensor(n - 4), 4, SCALE, nqh, nkvh, n_ctx)
+    torch.cuda.synchronize()
+    assert_close(o[:first].cpu().numpy(), ref[:first], "rows before the infinite scale")
+    assert torch.isnan(o[first:]).all()
+    assert torch.isnan(o4).all()
+    assert q27.device_status() == 0
