@@ -334,9 +334,10 @@ int q27b_prefill_row_plan(int M, int nkvh, int n_sm, int depth_hint, int must_me
 int q27b_prefill_split_plan(int M, int nqh, int n_sm, int depth_hint, int* split_tiles, int* pieces);
 
 /* Test hook for the failure path, no counterpart in the reference: launches one warp that waits on
- * a barrier nobody arrives at, with the bounded wait every kernel of this library uses. After the
- * limit (about two seconds) the wait gives up, the kernel returns normally and
- * q27b_device_status reports bit 0 (wait expired); the context stays usable. */
+ * a barrier nobody arrives at, with the bounded wait of this library's kernels (the int8 prefill kernel
+ * has a form of its own that counts polls: 17 s). After the limit (two to five seconds) the wait gives
+ * up, the kernel returns normally and q27b_device_status reports bit 0 (wait expired); the context stays
+ * usable. */
 int q27b_debug_expire_wait(void* stream);
 
 /* Measurement hook, no counterpart in the reference: while `event` (a cudaEvent_t) is set, every
