@@ -59,20 +59,25 @@ struct Geo {
   static constexpr int SC_BYTES = Q8 ? TILE * 16 : 0;
   static constexpr int STAGE_BYTES = 2 * VAL_BYTES + 2 * SC_BYTES;  // 34816 (q8_0) / 65536 (f16)
   static constexpr int NSTAGE = Q8 ? Q27B_NSTAGE : 3;
+  // Barriers "tile has landed": one for each stage and tile group that meet, tile t on barrier t % NFULL. With an odd
+  // number of stages a stage passes from one group to the other; on one barrier for both, a group that runs ahead could
+  // come to wait for its tile while the other group's tile before it has not landed, and its parity would be the
+  // barrier's already. On a barrier of its own a group waits for every tile in turn.
+  static constexpr int NFULL = NSTAGE % NGROUP == 0 ? NSTAGE : NSTAGE * NGROUP;
   static constexpr int OFF_KV = 0, OFF_VV = VAL_BYTES, OFF_KS = 2 * VAL_BYTES, OFF_VS = 2 * VAL_BYTES + SC_BYTES;
 };
 constexpr int RING_BYTES = Geo<true>::NSTAGE * Geo<true>::STAGE_BYTES > Geo<false>::NSTAGE * Geo<false>::STAGE_BYTES
                                ? Geo<true>::NSTAGE * Geo<true>::STAGE_BYTES
                                : Geo<false>::NSTAGE * Geo<false>::STAGE_BYTES;
-constexpr int MAX_STAGES = Geo<true>::NSTAGE > Geo<false>::NSTAGE ? Geo<true>::NSTAGE : Geo<false>::NSTAGE;
+constexpr int MAX_FULL = Geo<true>::NFULL > Geo<false>::NFULL ? Geo<true>::NFULL : Geo<false>::NFULL;
 constexpr int P_STRIDE = 36;                   // words per P row (32 position pairs + 4 padding: no bank conflicts)
 constexpr int P_WORDS = MAXR * P_STRIDE;
 constexpr int OFF_P = RING_BYTES;                           // [groups][2 buffers][24][36] words
 constexpr int OFF_MAX = OFF_P + NGROUP * 2 * P_WORDS * 4;   // [groups][2 buffers][4 warps][24] floats
 constexpr int OFF_L = OFF_MAX + NGROUP * 2 * 4 * MAXR * 4;  // [groups][4 warps][24] floats
 constexpr int OFF_M1 = OFF_L + NGROUP * 4 * MAXR * 4;       // [groups][24] floats: reference maxima at the end
-constexpr int OFF_BAR = OFF_M1 + NGROUP * MAXR * 4;         // full[stages]
-constexpr int OFF_FLAG = OFF_BAR + MAX_STAGES * 8;
+constexpr int OFF_BAR = OFF_M1 + NGROUP * MAXR * 4;         // full[MAX_FULL]
+constexpr int OFF_FLAG = OFF_BAR + MAX_FULL * 8;
 constexpr int OFF_TOK = OFF_FLAG + 16;                      // [groups][2 buffers] words: "move the maxima" tokens
 constexpr int SMEM_USED = OFF_TOK + 32;
 constexpr float TAU = 8.0f;                                 // a score may exceed the reference max by this much
@@ -134,7 +139,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constant__
               const __grid_constant__ CUtensorMap tm_vv, const __grid_constant__ CUtensorMap tm_vs,
               const DecodeParams p) {
   using G = Geo<Q8>;
-  constexpr int NSTAGE = G::NSTAGE;
+  constexpr int NSTAGE = G::NSTAGE, NFULL = G::NFULL;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sgen = smem_raw + (sbase - smem_u32(smem_raw));
@@ -149,7 +154,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constant__
       tma_prefetch_desc(&tm_ks);
       tma_prefetch_desc(&tm_vs);
     }
-    for (int s = 0; s < NSTAGE; s++) mbar_init(&full[s], 1);
+    for (int s = 0; s < NFULL; s++) mbar_init(&full[s], 1);
     *abort_flag = 0;
     for (int i = 0; i < 2 * NGROUP; i++) ((volatile uint32_t*)(sgen + OFF_TOK))[i] = 0;
     mbar_fence_init();
@@ -191,9 +196,9 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constant__
   // TMA of tile `it` into stage it % NSTAGE (one thread).
   const int row0 = kh * p.n_ctx + c0;
   auto issue_tile = [&](int it) {
-    const int s = it % NSTAGE;
-    uint8_t* st = sgen + (size_t)s * G::STAGE_BYTES;
-    mbar_expect_tx(&full[s], G::STAGE_BYTES);
+    uint8_t* st = sgen + (size_t)(it % NSTAGE) * G::STAGE_BYTES;
+    uint64_t* bar = &full[it % NFULL];
+    mbar_expect_tx(bar, G::STAGE_BYTES);
     int row = row0 + it * TILE;
     if (PAGED) {  // a tile never straddles a page (64 | 256)
       const int pp = c0 + it * TILE;
@@ -206,12 +211,12 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constant__
     }
 #pragma unroll
     for (int sg = 0; sg < G::NSEG; sg++) {
-      tma_load_2d(st + G::OFF_KV + sg * G::SEG_BYTES, &tm_kv, 128 * sg, row, &full[s]);
-      tma_load_2d(st + G::OFF_VV + sg * G::SEG_BYTES, &tm_vv, 128 * sg, row, &full[s]);
+      tma_load_2d(st + G::OFF_KV + sg * G::SEG_BYTES, &tm_kv, 128 * sg, row, bar);
+      tma_load_2d(st + G::OFF_VV + sg * G::SEG_BYTES, &tm_vv, 128 * sg, row, bar);
     }
     if (Q8) {
-      tma_load_2d(st + G::OFF_KS, &tm_ks, 0, row, &full[s]);
-      tma_load_2d(st + G::OFF_VS, &tm_vs, 0, row, &full[s]);
+      tma_load_2d(st + G::OFF_KS, &tm_ks, 0, row, bar);
+      tma_load_2d(st + G::OFF_VS, &tm_vs, 0, row, bar);
     }
   };
 
@@ -283,21 +288,10 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constant__
   const uint32_t vC = vQ + (vrow + 1) * 128 + ((vcb ^ ((vrow + 1) & 7)) << 4);
   const uint32_t sA = G::OFF_VS + (2 * wq + (g >> 2)) * 2 + vrow * 16;
 
-  if (NSTAGE % NGROUP != 0 && ntiles > NSTAGE) {
-    // With an odd number of stages a stage passes from one group to the other. A group must not come to wait for the
-    // second tile of a stage while the first one, the other group's, has not landed: the parity of that wait is then
-    // already the barrier's. Later tiles are safe, since each is requested by the other group from inside its tile; the
-    // first ones are requested at once. So nobody starts before tiles 0 and 1 are there (nothing is requested before
-    // either, and a barrier that had moved on twice could not be asked).
-    mbar_wait(&full[0], 0, abort_flag, p.status);
-    mbar_wait(&full[1], 0, abort_flag, p.status);
-    bar_sync(BAR_ALL, N_THREADS);
-  }
   int jt = 0;
   for (int it = grp; it < ntiles; it += NGROUP, jt++) {
-    const int s = it % NSTAGE;
-    mbar_wait(&full[s], (it / NSTAGE) & 1, abort_flag, p.status);
-    const uint32_t st = sbase + s * G::STAGE_BYTES;
+    mbar_wait(&full[it % NFULL], (it / NFULL) & 1, abort_flag, p.status);
+    const uint32_t st = sbase + (it % NSTAGE) * G::STAGE_BYTES;
     const int tile_p0 = c0 + it * TILE;
     const bool edge = tile_p0 + TILE > lim_min;  // some row of the tile is masked for some query row
 
