@@ -12,6 +12,7 @@ import ctypes
 import importlib.machinery
 import importlib.util
 import os
+import sysconfig
 
 import torch
 
@@ -101,6 +102,14 @@ def _load_binding():
     path = os.path.join(_HERE, "q27b_binding.so")
     if not os.path.exists(path):
         raise ImportError("q27b_binding.so is not built (run `python qwen27-engine_b200/build.py`); there is no fallback path")
+    # It is compiled against torch's C++ and Python's C interface: build.py leaves a note of which.
+    key = "torch %s, CXX11 ABI %d, %s" % (torch.__version__, torch._C._GLIBCXX_USE_CXX11_ABI, sysconfig.get_config_var("SOABI"))
+    note = os.path.join(_HERE, "build", "binding.key")
+    if os.path.exists(note):
+        with open(note) as f:
+            built = f.read()
+        if built != key:
+            raise ImportError("q27b_binding.so was built for %s, this is %s (run `python qwen27-engine_b200/build.py`)" % (built, key))
     loader = importlib.machinery.ExtensionFileLoader("q27b_binding", path)
     mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("q27b_binding", loader))
     loader.exec_module(mod)

@@ -17,6 +17,7 @@ OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libq27b_attn.so")
 SOURCES = ["host.cu", "kv_append.cu", "kv_wire.cu", "combine.cu", "decode.cu", "decode_tc.cu", "decode_ws.cu", "decode_wt.cu", "decode_ref.cu", "prefill.cu", "prefill_f16.cu", "sum_norm.cu", "peak_mma.cu", "pager.cu"]
 BINDING = os.path.join(HERE, "q27b_binding.so")
+BINDING_SOURCES = [os.path.join(CSRC, "binding.cpp"), os.path.join(HERE, "..", "include", "q27b_attn.h")]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
          "--expt-relaxed-constexpr"]
@@ -47,9 +48,23 @@ def _compile(src, verbose):
     return obj, r.stderr
 
 
+def binding_key():
+    """What a binary of the binding belongs to: it uses the C++ interface of torch and the C interface of this Python."""
+    import torch
+    return "torch %s, CXX11 ABI %d, %s" % (torch.__version__, torch._C._GLIBCXX_USE_CXX11_ABI, sysconfig.get_config_var("SOABI"))
+
+
+def _binding_stale():
+    try:
+        with open(os.path.join(OBJ, "binding.key")) as f:
+            key = f.read()
+    except OSError:
+        return True
+    return key != binding_key() or _stale(BINDING, BINDING_SOURCES)
+
+
 def _build_binding():
-    src = os.path.join(CSRC, "binding.cpp")
-    if not _stale(BINDING, [src]):
+    if not _binding_stale():
         return
     import torch
     root = os.path.dirname(torch.__file__)
@@ -60,10 +75,12 @@ def _build_binding():
            "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI]
     for d in inc:
         cmd += ["-isystem", d]
-    r = subprocess.run(cmd + [src, "-o", BINDING, "-L" + lib, "-Wl,-rpath," + lib, "-lc10", "-lc10_cuda", "-ltorch_cpu",
-                              "-ltorch_python"], capture_output=True, text=True)
+    r = subprocess.run(cmd + [BINDING_SOURCES[0], "-o", BINDING, "-L" + lib, "-Wl,-rpath," + lib, "-lc10", "-lc10_cuda",
+                              "-ltorch_cpu", "-ltorch_python"], capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("binding.cpp failed:\n%s\n%s" % (r.stdout, r.stderr))
+    with open(os.path.join(OBJ, "binding.key"), "w") as f:
+        f.write(binding_key())
 
 
 def build(verbose=False, force=False):

@@ -279,3 +279,26 @@ def test_binding_state_belongs_to_the_package_object(q27):
         with pytest.raises(m.Q27Error) as e:
             m.attn_decode(t, 0, 0, 0, 0, None, None, 0, 4, 0.1, 24, 4, 100)
         assert not isinstance(e.value, n.Q27Error)
+
+
+def test_binding_is_rebuilt_when_what_it_was_built_for_changes(q27, monkeypatch, tmp_path):
+    """Another torch, ABI or Python, a change of the public header, or an emptied build folder (--force) make the binary
+    stale; the package refuses one that was built for something else instead of loading it."""
+    import __graft_entry__ as ge
+    b = ge._load_build_module()
+    b.build()
+    assert not b._binding_stale()
+    with monkeypatch.context() as m:
+        m.setattr(torch, "__version__", "0.0.1")
+        assert b._binding_stale()
+        with pytest.raises(ImportError, match="built for torch"):
+            q27._load_binding()
+    with monkeypatch.context() as m:
+        m.setattr(b, "OBJ", str(tmp_path))
+        assert b._binding_stale()
+    assert any(s.endswith("q27b_attn.h") for s in b.BINDING_SOURCES)
+    newer = tmp_path / "header.h"
+    newer.write_text("")
+    os.utime(newer, (2 ** 31, 2 ** 31))
+    monkeypatch.setattr(b, "BINDING_SOURCES", b.BINDING_SOURCES + [str(newer)])
+    assert b._binding_stale()
