@@ -63,20 +63,29 @@ def _binding_stale():
     return key != binding_key() or _stale(BINDING, BINDING_SOURCES)
 
 
+def _torch_root():
+    import torch
+    return os.path.dirname(torch.__file__)
+
+
+def binding_compile(header_dir=os.path.dirname(BINDING_SOURCES[1])):
+    """The compiler and its language options and include folders."""
+    import torch
+    cmd = [os.environ.get("CXX", "g++"), "-std=c++17", "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI,
+           "-I", header_dir]
+    inc = os.path.join(_torch_root(), "include")
+    for d in (inc, os.path.join(inc, "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"], "/usr/local/cuda/include"):
+        cmd += ["-isystem", d]
+    return cmd
+
+
 def _build_binding():
     if not _binding_stale():
         return
-    import torch
-    root = os.path.dirname(torch.__file__)
-    lib = os.path.join(root, "lib")
-    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
-           sysconfig.get_paths()["include"], "/usr/local/cuda/include"]
-    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC",
-           "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI]
-    for d in inc:
-        cmd += ["-isystem", d]
-    r = subprocess.run(cmd + [BINDING_SOURCES[0], "-o", BINDING, "-L" + lib, "-Wl,-rpath," + lib, "-lc10", "-lc10_cuda",
-                              "-ltorch_cpu", "-ltorch_python"], capture_output=True, text=True)
+    lib = os.path.join(_torch_root(), "lib")
+    r = subprocess.run(binding_compile() + ["-O2", "-shared", "-fPIC", BINDING_SOURCES[0], "-o", BINDING, "-L" + lib,
+                                            "-Wl,-rpath," + lib, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"],
+                       capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("binding.cpp failed:\n%s\n%s" % (r.stdout, r.stderr))
     with open(os.path.join(OBJ, "binding.key"), "w") as f:

@@ -11,6 +11,8 @@
 
 #include <cstdint>
 
+#include "q27b_attn.h"
+
 namespace {
 
 enum Fn { PREP, DECODE, PREP_PAGED, DECODE_PAGED, PREFILL, N_FN };
@@ -86,9 +88,15 @@ PyObject* guarded(PyObject* self, Py_ssize_t n, Py_ssize_t want, B body) {
 }
 void* stream() { return (void*)c10::cuda::getCurrentCUDAStream().stream(); }
 
-#define PTR(i, type, opt, name) \
-  void* name;                   \
-  if (!ptr(st, a[i], type, opt, &name)) return nullptr
+template <c10::ScalarType T> struct Elem { using type = void; };
+template <> struct Elem<F32> { using type = float; };
+template <> struct Elem<I32> { using type = int; };
+template <> struct Elem<I8> { using type = int8_t; };
+
+#define PTR(i, kind, opt, name)                            \
+  void* name##_p;                                          \
+  if (!ptr(st, a[i], kind, opt, &name##_p)) return nullptr; \
+  Elem<kind>::type* name = static_cast<Elem<kind>::type*>(name##_p)
 #define NUM(i, name) \
   int name;          \
   if (!num(a[i], &name)) return nullptr
@@ -98,12 +106,13 @@ void* stream() { return (void*)c10::cuda::getCurrentCUDAStream().stream(); }
 #define FLAG(i, name) \
   int name;           \
   if (!flag(a[i], &name)) return nullptr
-#define CALL(which, type, ...)             \
-  void* s = stream();                \
-  int rc;                            \
-  Py_BEGIN_ALLOW_THREADS             \
-  rc = ((type)st->fn[which])(__VA_ARGS__); \
-  Py_END_ALLOW_THREADS               \
+// The signature is the header's: a parameter added, taken out or of another type there does not compile here.
+#define CALL(which, entry, ...)                                        \
+  void* s = stream();                                                  \
+  int rc;                                                              \
+  Py_BEGIN_ALLOW_THREADS                                               \
+  rc = reinterpret_cast<decltype(&entry)>(st->fn[which])(__VA_ARGS__); \
+  Py_END_ALLOW_THREADS                                                 \
   return done(st, rc)
 
 // qg, k, v, q_norm, k_norm, qn, kcache, vcache, pos0, T, eps, theta_scale, nqh, nkvh, n_ctx, q8, rope3, rdelta
@@ -113,8 +122,7 @@ PyObject* attn_prep(PyObject* self, PyObject* const* a, Py_ssize_t n) {
     PTR(5, F32, false, qn); PTR(6, ANY, false, kc); PTR(7, ANY, false, vc); PTR(8, I32, false, pos0);
     NUM(9, T); FLT(10, eps); FLT(11, theta); NUM(12, nqh); NUM(13, nkvh); NUM(14, n_ctx); FLAG(15, q8);
     PTR(16, I32, true, rope3); PTR(17, I32, true, rdelta);
-    using F = int (*)(void*, void*, void*, void*, void*, void*, void*, void*, void*, int, float, float, int, int, int, int, void*, void*, void*);
-    CALL(PREP, F, qg, k, v, qw, kw, qn, kc, vc, pos0, T, eps, theta, nqh, nkvh, n_ctx, q8, s, rope3, rdelta);
+    CALL(PREP, q27b_attn_prep, qg, k, v, qw, kw, qn, kc, vc, pos0, T, eps, theta, nqh, nkvh, n_ctx, q8, s, rope3, rdelta);
   });
 }
 
@@ -124,8 +132,7 @@ PyObject* attn_decode(PyObject* self, PyObject* const* a, Py_ssize_t n) {
     PTR(0, F32, false, qn); PTR(1, F32, false, qg); PTR(2, ANY, false, kc); PTR(3, ANY, false, vc); PTR(4, F32, true, o);
     PTR(5, I8, true, xq); PTR(6, F32, true, xd); PTR(7, I32, false, pos0);
     NUM(8, T); FLT(9, scale); NUM(10, nqh); NUM(11, nkvh); NUM(12, n_ctx); FLAG(13, q8);
-    using F = int (*)(void*, void*, void*, void*, void*, void*, void*, void*, int, float, int, int, int, int, void*);
-    CALL(DECODE, F, qn, qg, kc, vc, o, xq, xd, pos0, T, scale, nqh, nkvh, n_ctx, q8, s);
+    CALL(DECODE, q27b_attn_decode, qn, qg, kc, vc, o, xq, xd, pos0, T, scale, nqh, nkvh, n_ctx, q8, s);
   });
 }
 
@@ -136,8 +143,7 @@ PyObject* attn_prep_paged(PyObject* self, PyObject* const* a, Py_ssize_t n) {
     PTR(5, F32, true, qn); PTR(6, ANY, false, kp); PTR(7, ANY, false, vp); PTR(8, I32, false, table); PTR(9, I32, false, lens);
     NUM(10, B); NUM(11, T); FLT(12, eps); FLT(13, theta); NUM(14, nqh); NUM(15, nkvh); NUM(16, n_pages); NUM(17, max_pages);
     PTR(18, I32, true, rope3); PTR(19, I32, true, rdelta);
-    using F = int (*)(void*, void*, void*, void*, void*, void*, void*, void*, void*, void*, int, int, float, float, int, int, int, int, void*, void*, void*);
-    CALL(PREP_PAGED, F, qg, k, v, qw, kw, qn, kp, vp, table, lens, B, T, eps, theta, nqh, nkvh, n_pages, max_pages, s, rope3, rdelta);
+    CALL(PREP_PAGED, q27b_attn_prep_paged, qg, k, v, qw, kw, qn, kp, vp, table, lens, B, T, eps, theta, nqh, nkvh, n_pages, max_pages, s, rope3, rdelta);
   });
 }
 
@@ -147,8 +153,7 @@ PyObject* attn_decode_paged(PyObject* self, PyObject* const* a, Py_ssize_t n) {
     PTR(0, F32, false, qn); PTR(1, F32, false, qg); PTR(2, ANY, false, kp); PTR(3, ANY, false, vp); PTR(4, I32, false, table);
     PTR(5, I32, false, lens); PTR(6, F32, false, o);
     NUM(7, B); NUM(8, T); FLT(9, scale); NUM(10, nqh); NUM(11, nkvh); NUM(12, n_pages); NUM(13, max_pages); NUM(14, max_len);
-    using F = int (*)(void*, void*, void*, void*, void*, void*, void*, int, int, float, int, int, int, int, int, void*);
-    CALL(DECODE_PAGED, F, qn, qg, kp, vp, table, lens, o, B, T, scale, nqh, nkvh, n_pages, max_pages, max_len, s);
+    CALL(DECODE_PAGED, q27b_attn_decode_paged, qn, qg, kp, vp, table, lens, o, B, T, scale, nqh, nkvh, n_pages, max_pages, max_len, s);
   });
 }
 
@@ -158,8 +163,7 @@ PyObject* attn_prefill(PyObject* self, PyObject* const* a, Py_ssize_t n) {
     PTR(0, F32, false, qn); PTR(1, F32, false, qg); PTR(2, ANY, false, kc); PTR(3, ANY, false, vc); PTR(4, F32, false, o);
     PTR(5, I32, false, pos0);
     NUM(6, M); FLT(7, scale); NUM(8, nqh); NUM(9, nkvh); NUM(10, n_ctx); FLAG(11, q8); NUM(12, depth);
-    using F = int (*)(void*, void*, void*, void*, void*, void*, int, float, int, int, int, int, void*, int);
-    CALL(PREFILL, F, qn, qg, kc, vc, o, pos0, M, scale, nqh, nkvh, n_ctx, q8, s, depth);
+    CALL(PREFILL, q27b_attn_prefill, qn, qg, kc, vc, o, pos0, M, scale, nqh, nkvh, n_ctx, q8, s, depth);
   });
 }
 

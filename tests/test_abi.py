@@ -302,3 +302,16 @@ def test_binding_is_rebuilt_when_what_it_was_built_for_changes(q27, monkeypatch,
     os.utime(newer, (2 ** 31, 2 ** 31))
     monkeypatch.setattr(b, "BINDING_SOURCES", b.BINDING_SOURCES + [str(newer)])
     assert b._binding_stale()
+
+
+def test_binding_does_not_compile_against_another_signature(tmp_path):
+    """The binding calls through the header's own function types: a parameter added there is a compile error."""
+    import subprocess
+    import __graft_entry__ as ge
+    b = ge._load_build_module()
+    text = open(b.BINDING_SOURCES[1]).read()
+    a = "const int* pos0, int M, float kq_scale"
+    assert text.count(a) >= 1
+    (tmp_path / "q27b_attn.h").write_text(text.replace(a, "const int* pos0, int M, int extra, float kq_scale"))
+    r = subprocess.run(b.binding_compile(str(tmp_path)) + ["-fsyntax-only", b.BINDING_SOURCES[0]], capture_output=True, text=True)
+    assert r.returncode != 0 and "too few arguments" in r.stderr
