@@ -183,8 +183,23 @@ PyObject* bind(PyObject* self, PyObject* args) {
 #define FAST(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
 PyMethodDef g_methods[] = {{"bind", bind, METH_VARARGS, nullptr}, FAST(attn_prep), FAST(attn_decode), FAST(attn_prep_paged),
                            FAST(attn_decode_paged), FAST(attn_prefill), {nullptr, nullptr, 0, nullptr}};
+// The objects of the state belong to the package that holds this module: a cycle for the collector.
+int traverse(PyObject* self, visitproc visit, void* arg) {
+  State* st = (State*)PyModule_GetState(self);
+  if (!st) return 0;
+  Py_VISIT(st->ptr); Py_VISIT(st->check); Py_VISIT(st->f32); Py_VISIT(st->i32); Py_VISIT(st->i8);
+  return 0;
+}
+int clear(PyObject* self) {
+  State* st = (State*)PyModule_GetState(self);
+  if (!st) return 0;
+  Py_CLEAR(st->ptr); Py_CLEAR(st->check); Py_CLEAR(st->f32); Py_CLEAR(st->i32); Py_CLEAR(st->i8);
+  return 0;
+}
+void release(void* self) { clear((PyObject*)self); }
+
 PyModuleDef_Slot g_slots[] = {{0, nullptr}};
-PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "q27b_binding", nullptr, sizeof(State), g_methods, g_slots, nullptr, nullptr, nullptr};
+PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "q27b_binding", nullptr, sizeof(State), g_methods, g_slots, traverse, clear, release};
 
 }  // namespace
 

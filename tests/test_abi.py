@@ -315,3 +315,21 @@ def test_binding_does_not_compile_against_another_signature(tmp_path):
     (tmp_path / "q27b_attn.h").write_text(text.replace(a, "const int* pos0, int M, int extra, float kq_scale"))
     r = subprocess.run(b.binding_compile(str(tmp_path)) + ["-fsyntax-only", b.BINDING_SOURCES[0]], capture_output=True, text=True)
     assert r.returncode != 0 and "too few arguments" in r.stderr
+
+
+def test_a_dropped_package_object_is_freed(q27):
+    """The binding's module object holds functions of the package, whose globals hold the binding: the collector sees that
+    cycle."""
+    import gc
+    import importlib.util
+    import weakref
+    path = os.path.join(os.path.dirname(q27.__file__), "__init__.py")
+    spec = importlib.util.spec_from_file_location("q27_dropped_load", path, submodule_search_locations=[os.path.dirname(path)])
+    other = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(other)
+    with pytest.raises(other.Q27Error):
+        other.attn_decode(torch.zeros(4), 0, 0, 0, 0, None, None, 0, 4, 0.1, 24, 4, 100)
+    error = weakref.ref(other.Q27Error)
+    del other, spec
+    gc.collect()
+    assert error() is None
