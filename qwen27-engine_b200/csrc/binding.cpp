@@ -47,11 +47,8 @@ bool ptr(const State* st, PyObject* o, c10::ScalarType want, bool optional, void
 }
 
 bool num(PyObject* o, int* out) {  // int(o), as ctypes takes it: the low 32 bits
-  PyObject* l = PyLong_CheckExact(o) ? (Py_INCREF(o), o) : PyNumber_Check(o) || PyUnicode_Check(o) ? PyObject_CallOneArg((PyObject*)&PyLong_Type, o) : nullptr;
-  if (!l) {
-    if (!PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "int() argument must be a number");
-    return false;
-  }
+  PyObject* l = PyLong_CheckExact(o) ? Py_NewRef(o) : PyObject_CallOneArg((PyObject*)&PyLong_Type, o);
+  if (!l) return false;
   *out = (int)PyLong_AsUnsignedLongMask(l);
   Py_DECREF(l);
   return !PyErr_Occurred();

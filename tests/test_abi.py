@@ -333,3 +333,11 @@ def test_a_dropped_package_object_is_freed(q27):
     del other, spec
     gc.collect()
     assert error() is None
+
+
+@pytest.mark.parametrize("T", [b"4", bytearray(b" 4 "), "4", 4.7, True])
+def test_numbers_are_taken_as_int_takes_them(q27, T):
+    """Whatever int() makes a number of is one: the next to object is the library's shape check, without a GPU torch's
+    stream before it, and neither raises a TypeError."""
+    with pytest.raises(RuntimeError):
+        q27.attn_decode(16, 16, 16, 16, 16, None, None, 16, T, 0.1, 23, 4, 100)
