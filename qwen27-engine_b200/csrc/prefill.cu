@@ -846,6 +846,40 @@ int prefill_setup(DeviceCtx* ctx) {
   return Q27B_OK;
 }
 
+// What q27b_prefill_split_plan answers: the reference's rule for tiles of 128 tokens of one head, and a tail split of the
+// same tiles. For callers that lay work out by such tiles; the launchers plan with plan_prefill_rows.
+//  * Few CTAs: every tile is split, enough CTAs for every SM and at least 2048 positions per split
+//    (src/attn.cu:945-951). Q27_ATTN_SPLIT forces this form (src/attn.cu:952).
+//  * More CTAs than SMs on a deep prefix (all CTAs about equally long): the CTAs beyond the last full
+//    wave would leave most SMs idle for a whole CTA time (384 CTAs on 148 SMs: 3 rounds for 2.6
+//    rounds of work). The unsplit CTAs are launched first and only the earliest ts tiles - as many
+//    CTAs as the remainder - are cut into ns pieces that fill the machine evenly at the end; ns is
+//    the count that minimises the modelled makespan. Only ts / tiles of the rows pay for a merge.
+SplitPlan plan_prefill_split(int tiles, int nqh, int n_sm, int M, int depth_hint) {
+  const int ctas = tiles * nqh;
+  int ns = 1;
+  const int ns_max = depth_hint >= 0 ? std::max(1, std::min(8, (depth_hint + M) / 2048)) : 1;
+  if (depth_hint >= 0) ns = std::max(1, std::min((2 * n_sm + ctas - 1) / ctas, ns_max));
+  SplitPlan forced;
+  if (forced_plan(tiles, false, &forced)) return forced;
+  if (ns > 1) return {tiles, ns};
+  const char* tail = getenv("Q27B_PREFILL_TAIL_SPLIT");
+  if ((tail && tail[0] == '0') || depth_hint < 4 * M || ctas <= n_sm || ctas % n_sm == 0 || ns_max < 2) return {0, 1};
+  const int ts = std::min(tiles, (ctas % n_sm + nqh - 1) / nqh);
+  const int U = ctas - ts * nqh, a = U / n_sm, b = U % n_sm;
+  double best = (double)((ctas + n_sm - 1) / n_sm);  // not splitting at all
+  int best_ns = 1;
+  for (int k = 2; k <= ns_max; k++) {
+    const long P = (long)ts * nqh * k, cap = b ? (long)(n_sm - b) * k : 0;
+    double t = a + (b ? 1.0 : 0.0);
+    if (P > cap) t += (double)((P - cap + n_sm - 1) / n_sm) / k;
+    t += k * 1400.0 / (depth_hint + M);  // per piece: Q tile, pipeline fill, partials, merge (measured at 32k and 148k)
+    if (t < best) best = t, best_ns = k;
+  }
+  if (tail && atoi(tail) > 1) best_ns = std::min(atoi(tail), ns_max);  // tuning: Q27B_PREFILL_TAIL_SPLIT=<pieces>
+  return best_ns > 1 ? SplitPlan{ts, best_ns} : SplitPlan{0, 1};
+}
+
 }  // namespace
 
 }  // namespace q27b
@@ -870,7 +904,7 @@ extern "C" {
 
 int q27b_prefill_split_plan(int M, int nqh, int n_sm, int depth_hint, int* split_tiles, int* pieces) {
   if (M < 1 || nqh < 1 || n_sm < 1 || !split_tiles || !pieces) return fail(Q27B_BAD_SHAPE, "prefill_split_plan: bad argument");
-  const SplitPlan sp = plan_prefill_split((M + QT - 1) / QT, nqh, n_sm, M, depth_hint, false);
+  const SplitPlan sp = plan_prefill_split((M + QT - 1) / QT, nqh, n_sm, M, depth_hint);
   *split_tiles = sp.ts;
   *pieces = sp.ns;
   return Q27B_OK;

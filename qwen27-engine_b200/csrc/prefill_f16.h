@@ -14,41 +14,13 @@ namespace q27b {
 struct SplitPlan {
   int ts, ns;
 };
-// The reference's rule for tiles of 128 tokens of one head, and a tail split of the same tiles (q27b_prefill_split_plan;
-// the launchers plan with plan_prefill_rows).
-//  * Few CTAs: every tile is split, enough CTAs for every SM and at least 2048 positions per split
-//    (src/attn.cu:945-951). Q27_ATTN_SPLIT forces this form (src/attn.cu:952).
-//  * More CTAs than SMs on a deep prefix (all CTAs about equally long): the CTAs beyond the last full
-//    wave would leave most SMs idle for a whole CTA time (384 CTAs on 148 SMs: 3 rounds for 2.6
-//    rounds of work). The unsplit CTAs are launched first and only the earliest ts tiles - as many
-//    CTAs as the remainder - are cut into ns pieces that fill the machine evenly at the end; ns is
-//    the count that minimises the modelled makespan. Only ts / tiles of the rows pay for a merge.
-inline SplitPlan plan_prefill_split(int tiles, int nqh, int n_sm, int M, int depth_hint, bool must_merge) {
-  const int ctas = tiles * nqh;
-  int ns = 1;
-  const int ns_max = depth_hint >= 0 ? std::max(1, std::min(8, (depth_hint + M) / 2048)) : 1;
-  if (depth_hint >= 0) ns = std::max(1, std::min((2 * n_sm + ctas - 1) / ctas, ns_max));
-  if (const char* e = getenv("Q27_ATTN_SPLIT")) {
-    const int f = atoi(e);
-    if (f > 0) return {f > 1 || must_merge ? tiles : 0, std::max(std::min(f, 64), must_merge ? 2 : 1)};
-  }
-  if (must_merge) return {tiles, std::max(ns, 2)};
-  if (ns > 1) return {tiles, ns};
-  const char* tail = getenv("Q27B_PREFILL_TAIL_SPLIT");
-  if ((tail && tail[0] == '0') || depth_hint < 4 * M || ctas <= n_sm || ctas % n_sm == 0 || ns_max < 2) return {0, 1};
-  const int ts = std::min(tiles, (ctas % n_sm + nqh - 1) / nqh);
-  const int U = ctas - ts * nqh, a = U / n_sm, b = U % n_sm;
-  double best = (double)((ctas + n_sm - 1) / n_sm);  // not splitting at all
-  int best_ns = 1;
-  for (int k = 2; k <= ns_max; k++) {
-    const long P = (long)ts * nqh * k, cap = b ? (long)(n_sm - b) * k : 0;
-    double t = a + (b ? 1.0 : 0.0);
-    if (P > cap) t += (double)((P - cap + n_sm - 1) / n_sm) / k;
-    t += k * 1400.0 / (depth_hint + M);  // per piece: Q tile, pipeline fill, partials, merge (measured at 32k and 148k)
-    if (t < best) best = t, best_ns = k;
-  }
-  if (tail && atoi(tail) > 1) best_ns = std::min(atoi(tail), ns_max);  // tuning: Q27B_PREFILL_TAIL_SPLIT=<pieces>
-  return best_ns > 1 ? SplitPlan{ts, best_ns} : SplitPlan{0, 1};
+// Q27_ATTN_SPLIT=<n> of the reference (src/attn.cu:952): every tile in n pieces.
+inline bool forced_plan(int tiles, bool must_merge, SplitPlan* plan) {
+  const char* e = getenv("Q27_ATTN_SPLIT");
+  const int f = e ? atoi(e) : 0;
+  if (f <= 0) return false;
+  *plan = {f > 1 || must_merge ? tiles : 0, std::max(std::min(f, 64), must_merge ? 2 : 1)};
+  return true;
 }
 
 // The query rows of a KV head are its M * 6 (token, head) pairs, token-major; a CTA takes 128 of them.
@@ -73,17 +45,15 @@ inline int split_tokens(int M, int ts) { return ts >= row_tiles(M) ? M : ts / 3 
 inline SplitPlan plan_prefill_rows(int M, int nkvh, int n_sm, int depth_hint, bool must_merge) {
   constexpr double C0 = 3.0, CP = 4.0, M0 = 2.0, MROW = 1.2e-3, MPART = 2.0e-4;
   const int rt = row_tiles(M), ctas = rt * nkvh;
-  if (const char* e = getenv("Q27_ATTN_SPLIT")) {
-    const int f = atoi(e);
-    if (f > 0) return {f > 1 || must_merge ? rt : 0, std::max(std::min(f, 64), must_merge ? 2 : 1)};
-  }
+  SplitPlan plan;
+  if (forced_plan(rt, must_merge, &plan)) return plan;
   if (depth_hint < 0) return must_merge ? SplitPlan{rt, 2} : SplitPlan{0, 1};
   const bool deep = depth_hint >= M;
   if (!must_merge && !deep && ctas > n_sm) return {0, 1};
   const double N = ((double)depth_hint + M) / 64, rows = (double)M * nkvh * PF_GQA;
   const int ns_max = std::max(2, std::min(64, (int)(N / 2)));  // two position tiles a piece at least
   auto rounds = [&](double n) { return std::ceil(n / n_sm - 1e-9); };
-  SplitPlan plan = must_merge ? SplitPlan{rt, 2} : SplitPlan{0, 1};
+  plan = must_merge ? SplitPlan{rt, 2} : SplitPlan{0, 1};
   double best = must_merge ? 1e300 : rounds(ctas) * (N + C0);
   for (int k = 2; k <= ns_max && (k == 2 || (int64_t)ctas * (k - 1) < 4 * n_sm); k++) {
     const double t = rounds((double)ctas * k) * (N / k + C0 + CP) + M0 + rows * (MROW + MPART * k);

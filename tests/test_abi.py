@@ -124,6 +124,28 @@ def test_prefill_row_plan(q27, monkeypatch):
     assert q27.prefill_row_plan(2048, 4, 148, 32768) == (96, 3)
 
 
+@pytest.mark.parametrize("args,plan", [
+    ((2048, 4, 148, 32768), (24, 5)), ((2048, 4, 148, 148000), (24, 5)), ((896, 4, 148, 3600), (6, 7)),  # tail split
+    ((131, 4, 148, 30011), (7, 5)), ((2048, 4, 148, 32768, True), (96, 2)),                            # every tile
+    ((2048, 4, 148, 0), (0, 1)), ((1000, 1, 148, 100), (0, 1))])
+def test_prefill_row_plan_of_the_shapes_that_matter(q27, monkeypatch, args, plan):
+    monkeypatch.delenv("Q27_ATTN_SPLIT", raising=False)
+    monkeypatch.delenv("Q27B_PREFILL_TAIL_SPLIT", raising=False)
+    assert q27.prefill_row_plan(*args) == plan
+    tiles, tail = (6 * args[0] + 127) // 128, 0 < plan[0] < (6 * args[0] + 127) // 128
+    monkeypatch.setenv("Q27B_PREFILL_TAIL_SPLIT", "0")
+    if tail:
+        assert q27.prefill_row_plan(*args)[0] in (0, tiles)
+        monkeypatch.setenv("Q27B_PREFILL_TAIL_SPLIT", "3")
+        assert q27.prefill_row_plan(*args) == (plan[0], 3)
+    else:
+        assert q27.prefill_row_plan(*args) == plan
+    monkeypatch.setenv("Q27_ATTN_SPLIT", "4")  # goes before the tail split
+    assert q27.prefill_row_plan(*args) == (tiles, 4)
+    monkeypatch.setenv("Q27_ATTN_SPLIT", "1")
+    assert q27.prefill_row_plan(*args) == ((tiles, 2) if len(args) == 5 else (0, 1))
+
+
 def test_sum_norm_entry_points_check_their_arguments(q27):
     """Argument checks of the sum_norm family come before any CUDA call."""
     lib = ctypes.CDLL(q27.LIB_PATH)
