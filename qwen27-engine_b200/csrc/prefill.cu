@@ -11,8 +11,9 @@
 //
 // One CTA = 128 rows of one KV head (TMEM lane = row) x one split of the positions, walking 64-position
 // tiles. The rows of a KV head are its M * 6 (token, head) pairs, token-major: a tile spans 22 tokens of all
-// six heads, so that only the last tile of a KV head has empty rows (tiles of 128 tokens of one head: 16 tokens
-// behind 30,000 took 293 us, now 64; 131 behind 30,011 521, now 274) and fewer position tiles are half masked.
+// six heads, so that only the last tile of a KV head has empty rows and fewer position tiles are half masked (against
+// tiles of 128 tokens of one head, with this change alone: 16 tokens behind 30,000 293 -> 64 us, 131 behind 30,011
+// 521 -> 274).
 // Roles (16 warps):
 //   warps 0-7   softmax, two warpgroups: both own the 128 rows (warp w and w+4 share TMEM lanes
 //               32(w%4)..), warpgroup 0 takes positions 0-31 of a tile, warpgroup 1 positions
@@ -259,11 +260,11 @@ prefill_i8_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_consta
   volatile int* abort_flag = (volatile int*)(sgen + OFF_MISC + 4);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // CTA order: the query tiles with the most positions first (src/attn.cu:567). tile_major: and that
-  // across all heads (block L = head L % nqh of tile rank L / nqh), which matters on a short prefix,
-  // where the tiles differ a lot in length and the longest tiles of the last heads would start last.
-  // Otherwise head by head (block L = tile rank L % n_tiles of head L / n_tiles), so that the CTAs
-  // that run at the same time stream the same K/V rows and share them in L2 (measured: 7 % at 32k).
+  // CTA order: the row tiles with the most positions first (src/attn.cu:567). tile_major: and that across
+  // the KV heads (block L = KV head L % nkvh of tile rank L / nkvh), which matters on a short prefix, where
+  // the tiles differ a lot in length and the longest tiles of the last heads would start last. Otherwise KV
+  // head by KV head (block L = tile rank L % ntl of KV head L / ntl), so that the CTAs that run at the same
+  // time stream the same K/V rows and share them in L2 (7 % at 32k, measured with tiles of one query head).
   // The unsplit CTAs (tiles >= ts) come first, then the pieces of the split tiles, split index slowest.
   int L = (int)blockIdx.x, z = 0, nsplit = 1, ntl = row_tiles(p.M) - p.ts, tile_base = p.ts;
   if (L >= ntl * p.nkvh) {

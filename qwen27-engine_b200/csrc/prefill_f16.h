@@ -36,12 +36,18 @@ inline int split_tokens(int M, int ts) { return ts >= row_tiles(M) ? M : ts / 3 
 //  * nothing is split;
 //  * every tile is split. Few rows behind a long prefix leave most SMs idle otherwise, and a second, partly filled
 //    round of CTAs costs as much as a full one: 131 tokens behind 30,011 are 28 tiles, 5 pieces each fill one round of
-//    148 SMs (274 us; 3 pieces 407, 10 pieces 293). The other end: 1,000 tokens of one KV head behind 100, 47 tiles of
-//    17 position tiles, 55 us unsplit and 85 in 3 pieces: the merge of 6,000 rows costs more than the idle SMs.
+//    148 SMs (235 us a pass; 4 pieces 276, 6 pieces 359, 10 pieces 249). The other end: 1,000 tokens of one KV head
+//    behind 100, 47 tiles of 17 position tiles, 64 us unsplit and 86 in 3 pieces: the merge of 6,000 rows costs more
+//    than the idle SMs.
 //  * tail split: more CTAs than SMs on a deep prefix. The unsplit CTAs are launched first; only the earliest ts tiles,
 //    as many CTAs as the last round would hold, are cut, and their pieces fill the machine evenly at the end. 2048
-//    tokens behind 32,768 / 148,000: 3,640 / 15,611 us unsplit, 3,363 / 13,741 with 5 pieces, 3,386 / 13,854 with 8.
+//    tokens behind 32,768 / 148,000: 3,105 / 13,279 us unsplit, 2,874 / 11,774 with 5 pieces, 2,896 / 11,798 with 8.
 // On a short prefix the tiles differ in length (the causal part): longest first, no split once there is a CTA per SM.
+// The constants were fitted to an earlier form of the int8 kernel, whose position tile took a seventh longer, and serve
+// the f16-QK kernel too, whose tile takes two thirds of the present one. Checked with the present kernels against forced
+// pieces on ten shapes (16 to 2,048 tokens behind 100 to 148,000; the times above are of the int8 kernel): the choice is
+// within 2 % of the best for the int8 kernel; the f16-QK kernel on 50 tokens behind 3,000 takes 37.5 us and 36.5 with 10
+// pieces instead of 12, on an f16 cache 36.5 and 35.0, elsewhere within 2 % too.
 inline SplitPlan plan_prefill_rows(int M, int nkvh, int n_sm, int depth_hint, bool must_merge) {
   constexpr double C0 = 3.0, CP = 4.0, M0 = 2.0, MROW = 1.2e-3, MPART = 2.0e-4;
   const int rt = row_tiles(M), ctas = rt * nkvh;

@@ -303,7 +303,7 @@ def test_prefill_tail_split(q27, orc, q8):
     positions and merged, the others write their result directly. Checked on the token ranges around
     the boundary between the two kinds and at the end of the chunk; the q8_1 form of the same call."""
     from qwen27_engine_b200 import synth
-    nkvh, pos0, M = 4, 3600, 896      # 7 tiles x 24 heads = 168 CTAs, prefix >= 4 M
+    nkvh, pos0, M = 4, 3600, 896      # 42 row tiles x 4 KV heads = 168 CTAs: 6 tiles (128 tokens) in 7 pieces
     nqh, n = nkvh * GQA, pos0 + M
     n_ctx = n + 9
     qn = synth.normal(synth.SEED_Q, (M, nqh, AD))
@@ -360,8 +360,9 @@ def test_prefill_f16_qk_on_q8_cache(q27, orc, pos0, M, depth_hint):
 def test_prefill_i8_magnitudes(q27, orc, qs, ks):
     """The int8 kernel reads block sums as subnormal floats and moves powers of two between the Q and the K scales: the
     ends of their ranges (K scales from f16 subnormals to near the largest f16, tiny Q) against the oracle, and scores
-    large enough to move the reference maxima on most tiles (qs = 30). Tolerance as everywhere: the arithmetic is exact up
-    to f32 rounding."""
+    large enough to move the reference maxima on most tiles (qs = 30). With qs = 1e-20 the softmax is uniform whatever the
+    scores are: that case shows that nothing of it turns into NaN or infinity. The bound is relative to the outputs' RMS
+    (below)."""
     from qwen27_engine_b200 import synth
     pos0, M, nkvh = 333, 40, 1
     nqh, n = nkvh * GQA, pos0 + M
