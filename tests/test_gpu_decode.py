@@ -384,3 +384,105 @@ def test_f16_cache_many_tiles_a_chunk(q27, orc, T):
         torch.cuda.synchronize()
         assert_close(o.cpu().numpy(), ref, "f16 T=%d n=%d" % (T, n))
     assert q27.device_status() == 0
+
+
+def _leave_nan_in_the_workspace(q27, nkvh):
+    nqh = nkvh * GQA
+    nan = torch.full((4, nqh, AD), float("nan"), device="cuda")
+    kc = q27.new_cache(nkvh, 80000)
+    q27.attn_decode(nan, torch.zeros((4, nqh, 512), device="cuda"), kc, kc, torch.empty_like(nan), None, None,
+                    pos_tensor(80000 - 4), 4, SCALE, nqh, nkvh, 80000)
+
+
+# 148 chunks of one KV head, 74 of two (the merge that shares a row out over CTAs): the last length with a chunk of one
+# tile each, the last without a pool, and the next ones
+@pytest.mark.parametrize("nkvh,n", [(1, 1), (1, 65), (1, 9472), (1, 9473), (1, 75776), (1, 75777), (2, 64), (2, 4736), (2, 4737),
+                                    (2, 37888), (2, 37889), (4, 2369), (4, 18945)])
+@pytest.mark.parametrize("q8", [True, False], ids=["q8", "f16"])
+def test_empty_chunks_leave_no_trace_in_any_merge(q27, orc, decode_kernel, nkvh, n, q8):
+    """As above for every form of the merge and for f16 caches, whose kernel cuts its chunks by a formula of its own."""
+    from qwen27_engine_b200 import synth
+    if not q8 and decode_kernel != 1:
+        pytest.skip("f16 caches have one kernel")
+    T, nqh, n_ctx = min(n, 2), nkvh * GQA, n + 9
+    _leave_nan_in_the_workspace(q27, nkvh)
+    qn, qg, kf, vf = synth.decode_inputs(T, nqh, nkvh, n)
+    kc_ref, vc_ref = orc.fill_cache(kf, vf, n_ctx, q8=q8)
+    o = torch.full((T, nqh, AD), float("nan"), device="cuda")
+    q27.attn_decode(dev(qn), dev(qg), poisoned_cache(q27, kc_ref, nkvh, n_ctx, n, q8), poisoned_cache(q27, vc_ref, nkvh, n_ctx, n, q8),
+                    o, None, None, pos_tensor(n - T), T, SCALE, nqh, nkvh, n_ctx, q8)
+    torch.cuda.synchronize()
+    assert_close(o.cpu().numpy(), orc.attn_ref(qn, qg, kc_ref, vc_ref, n - T, SCALE, nkvh, n_ctx, q8=q8), "nkvh=%d n=%d" % (nkvh, n))
+    assert q27.device_status() == 0
+
+
+@pytest.mark.parametrize("nkvh", [1, 2, 4])
+@pytest.mark.parametrize("n_local", [0, 1, 65])
+def test_partial_of_a_short_slice_has_no_trace(q27, orc, nkvh, n_local):
+    """A slice of no, one or 65 rows of a longer sequence behind a workspace full of NaN: an empty slice is the neutral
+    partial, and merged with the rest of the sequence every slice gives the whole."""
+    from qwen27_engine_b200 import synth
+    T, n, nqh = 2, 700, nkvh * GQA
+    cut = n - n_local
+    qn, qg, kf, vf = synth.decode_inputs(T, nqh, nkvh, n)
+    rows, parts = T * nqh, []
+    for lo, hi in ((0, cut), (cut, n)):
+        n_ctx = max(hi - lo, 1) + 7
+        a, b = (lo, hi) if hi > lo else (0, 1)  # rows of an empty slice's cache: anything
+        kc_ref, vc_ref = orc.fill_cache(kf[:, a:b], vf[:, a:b], n_ctx)
+        kc, vc = poisoned_cache(q27, kc_ref, nkvh, n_ctx, hi - lo), poisoned_cache(q27, vc_ref, nkvh, n_ctx, hi - lo)
+        _leave_nan_in_the_workspace(q27, nkvh)
+        part = torch.full((T, nqh, 258), float("nan"), device="cuda")
+        q27.attn_decode_partial(dev(qn), kc, vc, part, pos_tensor(n - T), T, SCALE, nqh, nkvh, n_ctx, lo, hi - lo)
+        parts.append(part)
+    torch.cuda.synchronize()
+    if n_local == 0:
+        assert bool((parts[1][..., 0] == -1e30).all()) and bool((parts[1][..., 1:] == 0).all())
+    o = torch.empty((T, nqh, AD), device="cuda")
+    q27.lse_merge(torch.stack(parts).contiguous(), 2, rows * 258, rows, dev(qg), o)
+    torch.cuda.synchronize()
+    kc_ref, vc_ref = orc.fill_cache(kf, vf, n)
+    assert_close(o.cpu().numpy(), orc.attn_ref(qn, qg, kc_ref, vc_ref, n - T, SCALE, nkvh, n), "slice of %d rows" % n_local)
+    assert q27.device_status() == 0
+
+
+def test_steps_on_two_streams_of_the_caller(q27, orc):
+    """Steps issued in turn on two streams that wait for one another, neither the default one: the kernels that start
+    early on one stream find what the other has written (cache rows, position, query, workspace). n stays below the tile
+    pool, so the outputs are the same bits as with a synchronise behind every call."""
+    from qwen27_engine_b200 import synth
+    T, nkvh, n0, steps = 2, 2, 300, 12
+    nqh, n_ctx = nkvh * GQA, 1000
+    eps, theta = 1e-6, 10000000.0 ** (-2.0 / 64)
+    _, _, kf, vf = synth.decode_inputs(T, nqh, nkvh, n_ctx)
+    kc_ref, vc_ref = orc.fill_cache(kf, vf, n_ctx)
+    w = torch.ones(AD, device="cuda")
+    qg = [dev(synth.normal(synth.SEED_Q, (T, nqh, 512), start=i * 7919)) for i in range(steps)]
+    k = [dev(synth.normal(synth.SEED_K, (T, nkvh, AD), start=i * 7919)) for i in range(steps)]
+    v = [dev(synth.normal(synth.SEED_V, (T, nkvh, AD), start=i * 7919)) for i in range(steps)]
+
+    def run(streams, sync):
+        kc, vc, pos = dev(kc_ref), dev(vc_ref), pos_tensor(n0)
+        qn, o = torch.empty((T, nqh, AD), device="cuda"), [torch.empty((T, nqh, AD), device="cuda") for _ in range(steps)]
+        torch.cuda.synchronize()
+        for i in range(steps):
+            s = streams[i % 2]
+            s.wait_stream(streams[(i + 1) % 2])
+            with torch.cuda.stream(s):
+                q27.attn_prep(qg[i], k[i], v[i], w, w, qn, kc, vc, pos, T, eps, theta, nqh, nkvh, n_ctx)
+                if sync:
+                    torch.cuda.synchronize()
+                q27.attn_decode(qn, qg[i], kc, vc, o[i], None, None, pos, T, SCALE, nqh, nkvh, n_ctx)
+                pos += T
+            if sync:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return o, kc, vc
+
+    d = torch.cuda.current_stream()
+    want = run((d, d), True)
+    for _ in range(3):
+        got = run((torch.cuda.Stream(), torch.cuda.Stream()), False)
+        assert all(torch.equal(a, b) for a, b in zip(got[0], want[0]))
+        assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
+    assert q27.device_status() == 0
