@@ -1,6 +1,6 @@
 // CPU restatement of the attention hot path of avallavall/qwen27-engine.
 //
-// TEST INFRASTRUCTURE ONLY. This file is the checker: tests, the smoke check and the
+// TEST INFRASTRUCTURE ONLY. This file is the oracle: tests, the smoke check and the
 // cpu_baseline leg of the benchmark call it. The shipped library never links or loads it.
 //
 // Parity status: the reference holds no golden vectors for this path (its only check,

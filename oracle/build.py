@@ -1,4 +1,4 @@
-"""Build recipes for the checker code (test infrastructure, never shipped).
+"""Build recipes for the oracle code (test infrastructure, never shipped).
 
 build_oracle(): oracle/attn_oracle.cpp -> oracle/liboracle.so (g++ -fopenmp).
 build_ref():    the reference's own src/attn.cu + src/ops.cu, compiled where they lie in the
