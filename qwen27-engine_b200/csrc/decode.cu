@@ -637,10 +637,10 @@ int kernel_choice() {
 }
 // Launches the split-K kernel chosen for a q8_0 cache.
 int launch_q8(const CUtensorMap* kv, const CUtensorMap* ks, const CUtensorMap* vv, const CUtensorMap* vs,
-              const DecodeParams& p, bool paged, int nseq, cudaStream_t s, bool single_group = false) {
+              const DecodeParams& p, bool paged, int nseq, cudaStream_t s, WsGroups groups = WsGroups::TWO) {
   const int k = kernel_choice();
   if (k == 2) return launch_decode_tc(kv, ks, vv, vs, p, paged, nseq, s);
-  if (k == 0 || k == 3) return launch_decode_ws(kv, ks, vv, vs, p, paged, nseq, s, single_group);
+  if (k == 0 || k == 3) return launch_decode_ws(kv, ks, vv, vs, p, paged, nseq, s, groups);
   if (k == 4) return launch_decode_wt(kv, ks, vv, vs, p, paged, nseq, s);
   return paged ? launch_decode_t<true, true>(kv, ks, vv, vs, p, nseq, s) : launch_decode_t<false, true>(kv, ks, vv, vs, p, nseq, s);
 }
@@ -967,7 +967,13 @@ int q27b_attn_decode_paged(const float* qn, const float* qg, const void* kpool, 
   p.T = T; p.nqh = nqh; p.nkvh = nkvh; p.n_ctx = max_pages * Q27B_PAGE; p.nch = nch; p.kq_scale = kq_scale;
   p.base_pos = 0; p.n_local = -1;
   p.page_table = page_table; p.seq_len = seq_len; p.max_pages = max_pages; p.n_pages = n_pages; p.chunk_len = chunk;
-  if (int rc = launch_q8(kv, ks, vv, vs, p, true, B, (cudaStream_t)stream, single_group)) return rc;
+  // A launch of no more CTAs than SMs must not put two on one: launched while the previous pass drains, its CTAs would go
+  // to the SMs that are free first, in pairs (two sequences of up to 15,751 positions, three tokens: 38.8 us a pass in
+  // pairs, 29.6 spread, 33.5 launched after the drain). From 149 CTAs on some SM has two in any case (ten sequences of
+  // up to 5,114: 44.0 us in pairs, 49.2 after the drain).
+  const bool spread = (int64_t)nch * nkvh * B <= ctx->n_sm;
+  const WsGroups groups = !single_group ? WsGroups::TWO : spread ? WsGroups::SPREAD : WsGroups::PAIRED;
+  if (int rc = launch_q8(kv, ks, vv, vs, p, true, B, (cudaStream_t)stream, groups)) return rc;
   MergeParams mp = {};
   mp.part = part; mp.nparts = nch; mp.rows = (int64_t)B * T * nqh; mp.qg = qg; mp.o = o; mp.T = T; mp.nqh = nqh;
   mp.seq_len = seq_len; mp.chunk_len = chunk;

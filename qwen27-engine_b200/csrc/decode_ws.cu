@@ -795,20 +795,25 @@ decode_ws_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constan
   if (tid == PV0) stamp(7);
 }
 
+// Shared memory of a CTA of one tile group that has an SM to itself: more than half of what an SM has.
+constexpr int SPREAD_SMEM_BYTES = 116 * 1024;
+static_assert(SPREAD_SMEM_BYTES >= Lay<1>::SMEM_BYTES && 2 * (SPREAD_SMEM_BYTES + 1024) > 228 * 1024, "one CTA per SM");
+
 template <int NT, int NG>
 int launch_ws_nt(const CUtensorMap* kv, const CUtensorMap* ks, const CUtensorMap* vv, const CUtensorMap* vs,
-                 const DecodeParams& p, bool paged, int nseq, cudaStream_t s) {
+                 const DecodeParams& p, bool paged, int nseq, cudaStream_t s, int smem = Lay<NG>::SMEM_BYTES) {
   const dim3 grid(p.nch, p.nkvh, nseq);
   if (paged)
-    Q27B_CK(launch_step(decode_ws_kernel<NT, true, NG>, grid, dim3(Lay<NG>::THREADS), Lay<NG>::SMEM_BYTES, s, *kv, *ks, *vv, *vs, p));
+    Q27B_CK(launch_step(decode_ws_kernel<NT, true, NG>, grid, dim3(Lay<NG>::THREADS), smem, s, *kv, *ks, *vv, *vs, p));
   else
-    Q27B_CK(launch_step(decode_ws_kernel<NT, false, NG>, grid, dim3(Lay<NG>::THREADS), Lay<NG>::SMEM_BYTES, s, *kv, *ks, *vv, *vs, p));
+    Q27B_CK(launch_step(decode_ws_kernel<NT, false, NG>, grid, dim3(Lay<NG>::THREADS), smem, s, *kv, *ks, *vv, *vs, p));
   return Q27B_OK;
 }
 
 template <int NT, bool PAGED, int NG>
 int ws_attr() {
-  Q27B_CK(cudaFuncSetAttribute(decode_ws_kernel<NT, PAGED, NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay<NG>::SMEM_BYTES));
+  Q27B_CK(cudaFuncSetAttribute(decode_ws_kernel<NT, PAGED, NG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               NG == 1 ? SPREAD_SMEM_BYTES : Lay<NG>::SMEM_BYTES));
   if (NG == 1)  // two CTAs per SM need the whole shared-memory carve-out
     Q27B_CK(cudaFuncSetAttribute(decode_ws_kernel<NT, PAGED, NG>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   return Q27B_OK;
@@ -830,7 +835,7 @@ int decode_ws_setup() {
 }
 
 int launch_decode_ws(const CUtensorMap* kv, const CUtensorMap* ks, const CUtensorMap* vv, const CUtensorMap* vs,
-                     const DecodeParams& p, bool paged, int nseq, cudaStream_t s, bool single_group) {
+                     const DecodeParams& p, bool paged, int nseq, cudaStream_t s, WsGroups groups) {
   static bool attr[64] = {};
   static std::mutex attr_mu;
   int dev;
@@ -843,10 +848,11 @@ int launch_decode_ws(const CUtensorMap* kv, const CUtensorMap* ks, const CUtenso
     }
   }
   const int nt = (GQA * p.T + 7) / 8;
-  if (single_group && paged) {  // 8 warps, two CTAs per SM
-    if (nt == 1) return launch_ws_nt<1, 1>(kv, ks, vv, vs, p, true, nseq, s);
-    if (nt == 2) return launch_ws_nt<2, 1>(kv, ks, vv, vs, p, true, nseq, s);
-    return launch_ws_nt<3, 1>(kv, ks, vv, vs, p, true, nseq, s);
+  if (groups != WsGroups::TWO && paged) {
+    const int smem = groups == WsGroups::SPREAD ? SPREAD_SMEM_BYTES : Lay<1>::SMEM_BYTES;
+    if (nt == 1) return launch_ws_nt<1, 1>(kv, ks, vv, vs, p, true, nseq, s, smem);
+    if (nt == 2) return launch_ws_nt<2, 1>(kv, ks, vv, vs, p, true, nseq, s, smem);
+    return launch_ws_nt<3, 1>(kv, ks, vv, vs, p, true, nseq, s, smem);
   }
   if (nt == 1) return launch_ws_nt<1, 2>(kv, ks, vv, vs, p, paged, nseq, s);
   if (nt == 2) return launch_ws_nt<2, 2>(kv, ks, vv, vs, p, paged, nseq, s);

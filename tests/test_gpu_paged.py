@@ -70,6 +70,12 @@ def test_paged_batched_decode(q27, orc, T, lens):
     assert q27.device_status() == 0
 
 
+@pytest.mark.parametrize("B", [74, 75])
+def test_paged_around_one_cta_per_sm(q27, orc, B):
+    """148 CTAs (an SM each) and 150 (in pairs) of one chunk each, over 2 KV heads."""
+    test_paged_batched_decode(q27, orc, 2, [2 + 13 * b % 700 for b in range(B)])
+
+
 def test_bad_page_is_flagged_not_followed(q27, orc):
     nkvh, nqh, T, n = 1, 6, 1, 300
     n_pages = 4
