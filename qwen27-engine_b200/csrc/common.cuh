@@ -156,6 +156,8 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* t
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
 }
+// Brings the line of a global address into L2.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // Byte offset of 16-byte chunk `chunk` (0..7) of 128-byte row `row` in a tile stored with the

@@ -168,6 +168,7 @@ prefill_f16_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   (void)VCONV_WARP0;
   constexpr int CW = PT / NWG;    // columns (positions) of a tile per softmax thread
   constexpr int OW = AD / NWG;    // columns of O per softmax thread (rescale, epilogue)
+  constexpr bool ROOM = LY::THREADS <= 384;  // registers for more loads in flight: 168 a thread; with 19 warps 96
   constexpr int NKF = LY::NKF, OFF_K = LY::OFF_K, OFF_V = LY::OFF_V, OFF_P = LY::OFF_P, OFF_RAW = LY::OFF_RAW,
                 OFF_XCH = LY::OFF_XCH, OFF_BAR = LY::OFF_BAR, OFF_MISC = LY::OFF_MISC;
   pdl_wait();
@@ -251,7 +252,17 @@ prefill_f16_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     const int t = (row0 + r) / GQA, h = kh * GQA + (row0 + r) % GQA;
     float* xch = (float*)(sgen + OFF_XCH);
     const uint32_t tlane = tmem + ((uint32_t)(q * 32) << 16);
+    // The gate is read at the very end, a round trip at a time, and nothing has touched it: into L2 now. This warp:
+    // OW / 32 lines of each of its rows.
+    if (nsplit == 1) {
+#pragma unroll
+      for (int i = 0; i < OW / 32; i++) {
+        const int gr = row0 + q * 32 + i * (1024 / OW) + lane / (OW / 32), tt = gr / GQA;
+        if (tt < p.M) prefetch_l2(p.qg + ((size_t)tt * p.nqh + kh * GQA + gr % GQA) * 512 + 256 + wg * OW + 32 * (lane % (OW / 32)));
+      }
+    }
     {
+      constexpr int LD = ROOM ? 2 : 1;  // turns whose loads are requested together
       // Q tile -> tensor memory, the A operand of every Q K^T MMA of this CTA (lane = row, column c =
       // dims 2c, 2c+1 as f16, even dim in the low half): it is read from there 16 times per tile
       // without touching shared memory. This warp writes dims OW wg .. OW wg + OW - 1 of its 32 rows,
@@ -265,30 +276,36 @@ prefill_f16_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         if (turn > 0) row_sync<NWG>(q);
         if ((wg >> 1) != turn) continue;
 #pragma unroll 1
-        for (; c < OW / 32; c++) {
-          float4 x[8];
+        for (; c < OW / 32; c += LD) {
+          float4 x[LD][8];
 #pragma unroll
-          for (int i = 0; i < 8; i++) {
-            const int gr = row0 + q * 32 + 4 * i + (lane >> 3), tt = gr / GQA;
-            x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (tt < p.M)
-              x[i] = *(const float4*)(p.qn + ((size_t)tt * p.nqh + kh * GQA + gr % GQA) * AD + OW * wg + c * 32 + 4 * (lane & 7));
-          }
+          for (int u = 0; u < LD; u++)
 #pragma unroll
-          for (int i = 0; i < 8; i++) {
-            const int rr = 4 * i + (lane >> 3), ch = ((lane & 7) >> 1) ^ ((rr >> 1) & 3);
-            *(uint2*)(stage + rr * 64 + ch * 16 + (lane & 1) * 8) =
-                make_uint2(pack_h2(x[i].x * p.kq_scale, x[i].y * p.kq_scale), pack_h2(x[i].z * p.kq_scale, x[i].w * p.kq_scale));
-          }
-          __syncwarp();
-          uint32_t w[16];
+            for (int i = 0; i < 8; i++) {
+              const int gr = row0 + q * 32 + 4 * i + (lane >> 3), tt = gr / GQA;
+              x[u][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (tt < p.M)
+                x[u][i] = *(const float4*)(p.qn + ((size_t)tt * p.nqh + kh * GQA + gr % GQA) * AD + OW * wg + (c + u) * 32 + 4 * (lane & 7));
+            }
 #pragma unroll
-          for (int i = 0; i < 4; i++) {
-            const uint4 u = *(const uint4*)(stage + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4));
-            w[4 * i] = u.x; w[4 * i + 1] = u.y; w[4 * i + 2] = u.z; w[4 * i + 3] = u.w;
+          for (int u = 0; u < LD; u++) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+              const int rr = 4 * i + (lane >> 3), ch = ((lane & 7) >> 1) ^ ((rr >> 1) & 3);
+              const float4 v = x[u][i];
+              *(uint2*)(stage + rr * 64 + ch * 16 + (lane & 1) * 8) =
+                  make_uint2(pack_h2(v.x * p.kq_scale, v.y * p.kq_scale), pack_h2(v.z * p.kq_scale, v.w * p.kq_scale));
+            }
+            __syncwarp();
+            uint32_t w[16];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+              const uint4 v = *(const uint4*)(stage + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4));
+              w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
+            }
+            tmem_st16(tlane + TM_Q + wg * (OW / 2) + (c + u) * 16, w);
+            __syncwarp();
           }
-          tmem_st16(tlane + TM_Q + wg * (OW / 2) + c * 16, w);
-          __syncwarp();
         }
       }
       tc_wait_st();
@@ -407,6 +424,26 @@ prefill_f16_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     row_sync<NWG>(q);
 #pragma unroll
     for (int o = 1; o < NWG; o++) l += xch[((nt & 1) * NWG + ((wg + o) % NWG)) * QT + r];
+    // Gate of 4 GB rows and 32 columns, requested together and ahead of the stores, which the compiler cannot move loads
+    // over: before the wait for O, then as soon as the last ones are used.
+    constexpr int GB = ROOM ? 8 : 4;
+    float4 gate[GB];
+    // Opaque to the compiler, so that it does not keep the addresses of all rows over the turns where that would spill.
+    auto first_row = [&]() {
+      int r0 = row0 + q * 32;
+      if (!ROOM) asm volatile("" : "+r"(r0));
+      return r0;
+    };
+    auto load_gate = [&](int c, int i0) {
+      if (nsplit > 1 || c == OW / 32) return;
+      const int r0 = first_row();
+#pragma unroll
+      for (int i = 0; i < GB; i++) {
+        const int gr = r0 + 4 * (i0 + i) + (lane >> 3), tt = gr / GQA;
+        if (tt < p.M) gate[i] = *(const float4*)(p.qg + ((size_t)tt * p.nqh + kh * GQA + gr % GQA) * 512 + 256 + wg * OW + c * 32 + 4 * (lane & 7));
+      }
+    };
+    load_gate(0, 0);
     mbar_wait(&bar[B_ODONE], 0, abort_flag, p.status);
     tc_fence_after();
     const float inv_l = 1.0f / l;
@@ -430,25 +467,30 @@ prefill_f16_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
                                                             __uint_as_float(v[4 * i + 2]) * f, __uint_as_float(v[4 * i + 3]) * f);
       }
       __syncwarp();
-#pragma unroll 4
-      for (int i = 0; i < 8; i++) {
-        const int rr = 4 * i + (lane >> 3), gr = row0 + q * 32 + rr, tt = gr / GQA;
-        if (tt >= p.M) continue;
-        const size_t th = (size_t)tt * p.nqh + kh * GQA + gr % GQA;
-        const int d = d0 + 4 * (lane & 7);
-        float4 y = *(const float4*)(stage + swz128(rr, lane & 7));
-        if (nsplit > 1) {
-          float* po = p.part + ((size_t)z * p.Ms * p.nqh + th) * PROW + 2 + d;
-          *(float2*)po = make_float2(y.x, y.y);
-          *(float2*)(po + 2) = make_float2(y.z, y.w);
-        } else {
-          const float4 gg = *(const float4*)(p.qg + th * 512 + 256 + d);
-          y.x *= 1.0f / (1.0f + __expf(-gg.x));
-          y.y *= 1.0f / (1.0f + __expf(-gg.y));
-          y.z *= 1.0f / (1.0f + __expf(-gg.z));
-          y.w *= 1.0f / (1.0f + __expf(-gg.w));
-          *(float4*)(p.o + th * AD + d) = y;
+#pragma unroll
+      for (int i0 = 0; i0 < 8; i0 += GB) {
+        const int r0 = first_row();
+#pragma unroll
+        for (int i = 0; i < GB; i++) {
+          const int rr = 4 * (i0 + i) + (lane >> 3), gr = r0 + rr, tt = gr / GQA;
+          if (tt >= p.M) continue;
+          const size_t th = (size_t)tt * p.nqh + kh * GQA + gr % GQA;
+          const int d = d0 + 4 * (lane & 7);
+          float4 y = *(const float4*)(stage + swz128(rr, lane & 7));
+          if (nsplit > 1) {
+            float* po = p.part + ((size_t)z * p.Ms * p.nqh + th) * PROW + 2 + d;
+            *(float2*)po = make_float2(y.x, y.y);
+            *(float2*)(po + 2) = make_float2(y.z, y.w);
+          } else {
+            const float4 gg = gate[i];
+            y.x *= 1.0f / (1.0f + __expf(-gg.x));
+            y.y *= 1.0f / (1.0f + __expf(-gg.y));
+            y.z *= 1.0f / (1.0f + __expf(-gg.z));
+            y.w *= 1.0f / (1.0f + __expf(-gg.w));
+            *(float4*)(p.o + th * AD + d) = y;
+          }
         }
+        load_gate(i0 + GB < 8 ? c : c + 1, i0 + GB < 8 ? i0 + GB : 0);
       }
       __syncwarp();
     }
