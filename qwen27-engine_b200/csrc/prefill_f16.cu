@@ -467,30 +467,34 @@ prefill_f16_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
                                                             __uint_as_float(v[4 * i + 2]) * f, __uint_as_float(v[4 * i + 3]) * f);
       }
       __syncwarp();
-#pragma unroll
-      for (int i0 = 0; i0 < 8; i0 += GB) {
-        const int r0 = first_row();
-#pragma unroll
-        for (int i = 0; i < GB; i++) {
-          const int rr = 4 * (i0 + i) + (lane >> 3), gr = r0 + rr, tt = gr / GQA;
+      if (nsplit > 1) {
+#pragma unroll 4
+        for (int i = 0; i < 8; i++) {
+          const int rr = 4 * i + (lane >> 3), gr = row0 + q * 32 + rr, tt = gr / GQA;
           if (tt >= p.M) continue;
-          const size_t th = (size_t)tt * p.nqh + kh * GQA + gr % GQA;
-          const int d = d0 + 4 * (lane & 7);
-          float4 y = *(const float4*)(stage + swz128(rr, lane & 7));
-          if (nsplit > 1) {
-            float* po = p.part + ((size_t)z * p.Ms * p.nqh + th) * PROW + 2 + d;
-            *(float2*)po = make_float2(y.x, y.y);
-            *(float2*)(po + 2) = make_float2(y.z, y.w);
-          } else {
+          const float4 y = *(const float4*)(stage + swz128(rr, lane & 7));
+          float* po = p.part + (((size_t)z * p.Ms + tt) * p.nqh + kh * GQA + gr % GQA) * PROW + 2 + d0 + 4 * (lane & 7);
+          *(float2*)po = make_float2(y.x, y.y);
+          *(float2*)(po + 2) = make_float2(y.z, y.w);
+        }
+      } else {
+#pragma unroll
+        for (int i0 = 0; i0 < 8; i0 += GB) {
+          const int r0 = first_row();
+#pragma unroll
+          for (int i = 0; i < GB; i++) {
+            const int rr = 4 * (i0 + i) + (lane >> 3), gr = r0 + rr, tt = gr / GQA;
+            if (tt >= p.M) continue;
+            float4 y = *(const float4*)(stage + swz128(rr, lane & 7));
             const float4 gg = gate[i];
             y.x *= 1.0f / (1.0f + __expf(-gg.x));
             y.y *= 1.0f / (1.0f + __expf(-gg.y));
             y.z *= 1.0f / (1.0f + __expf(-gg.z));
             y.w *= 1.0f / (1.0f + __expf(-gg.w));
-            *(float4*)(p.o + th * AD + d) = y;
+            *(float4*)(p.o + ((size_t)tt * p.nqh + kh * GQA + gr % GQA) * AD + d0 + 4 * (lane & 7)) = y;
           }
+          load_gate(i0 + GB < 8 ? c : c + 1, i0 + GB < 8 ? i0 + GB : 0);
         }
-        load_gate(i0 + GB < 8 ? c : c + 1, i0 + GB < 8 ? i0 + GB : 0);
       }
       __syncwarp();
     }
