@@ -322,8 +322,9 @@ int q27b_set_prefill_kernel(int which);
 /* How a q27b_attn_prefill call of M tokens and nkvh KV heads (6 nkvh query heads) on a GPU of n_sm SMs shares
  * out its work (host arithmetic only, no GPU needed). The query rows of a KV head are its M * 6 (token, head)
  * pairs, token-major, cut into tiles of 128 rows; the first *split_tiles tiles of every KV head are cut into
- * *pieces pieces over their positions (partials + merge), the others are not. 0 / 1 = no split. must_merge: the
- * plan of a call whose output the merge writes (q8_1 from the f16-QK kernel): every tile is split. */
+ * *pieces pieces over their positions (partials + merge), the others are not. 0 / 1 = no split. The plan of
+ * the int8 kernel; must_merge: of a call whose output the merge writes (q8_1 from the f16-QK kernel): every tile
+ * is split. (The f16-QK kernel's other calls count a merged row as dearer, and split less of a short prefix.) */
 int q27b_prefill_row_plan(int M, int nkvh, int n_sm, int depth_hint, int must_merge, int* split_tiles, int* pieces);
 
 /* The same for query tiles of 128 tokens of one head, as the reference tiles a chunk (its rule of splitting;

@@ -913,7 +913,7 @@ int q27b_prefill_split_plan(int M, int nqh, int n_sm, int depth_hint, int* split
 
 int q27b_prefill_row_plan(int M, int nkvh, int n_sm, int depth_hint, int must_merge, int* split_tiles, int* pieces) {
   if (M < 1 || nkvh < 1 || n_sm < 1 || !split_tiles || !pieces) return fail(Q27B_BAD_SHAPE, "prefill_row_plan: bad argument");
-  const SplitPlan sp = plan_prefill_rows(M, nkvh, n_sm, depth_hint, must_merge != 0);
+  const SplitPlan sp = plan_prefill_rows(M, nkvh, n_sm, depth_hint, must_merge != 0, must_merge != 0);
   *split_tiles = sp.ts;
   *pieces = sp.ns;
   return Q27B_OK;
@@ -939,7 +939,7 @@ static int prefill_impl(const float* qn, const float* qg, const void* kcache, co
   if (int rc = prefill_setup(ctx)) return rc;
   cudaStream_t s = (cudaStream_t)stream;
   const int tiles = row_tiles(M);
-  SplitPlan sp = plan_prefill_rows(M, nkvh, ctx->n_sm, depth_hint, false);
+  SplitPlan sp = plan_prefill_rows(M, nkvh, ctx->n_sm, depth_hint, false, false);
   float* part;  // the fixed prefill workspace; the plan is cut to what it holds
   if (int rc = fit_prefill_split(ctx, &sp.ts, &sp.ns, split_tokens(M, sp.ts), nqh, false, &part)) return rc;
   const int nsplit = sp.ns, Ms = split_tokens(M, sp.ts);

@@ -639,7 +639,7 @@ int launch_prefill_f16(DeviceCtx* ctx, const float* qn, const float* qg, const v
   const int tiles = row_tiles(M);
   // splits over the positions as for the int8 kernel; the q8_1 output is written by the merge kernel,
   // so it needs every tile on the split path (at least one merge)
-  SplitPlan sp = plan_prefill_rows(M, nkvh, ctx->n_sm, depth_hint, xq != nullptr);
+  SplitPlan sp = plan_prefill_rows(M, nkvh, ctx->n_sm, depth_hint, xq != nullptr, true);
   float* part;  // the fixed prefill workspace; the plan is cut to what it holds
   if (int rc = fit_prefill_split(ctx, &sp.ts, &sp.ns, split_tokens(M, sp.ts), nqh, xq != nullptr, &part)) return rc;
   const int nsplit = sp.ns, Ms = split_tokens(M, sp.ts);

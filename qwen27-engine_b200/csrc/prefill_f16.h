@@ -43,13 +43,17 @@ inline int split_tokens(int M, int ts) { return ts >= row_tiles(M) ? M : ts / 3 
 //    as many CTAs as the last round would hold, are cut, and their pieces fill the machine evenly at the end. 2048
 //    tokens behind 32,768 / 148,000: 3,105 / 13,279 us unsplit, 2,874 / 11,774 with 5 pieces, 2,896 / 11,798 with 8.
 // On a short prefix the tiles differ in length (the causal part): longest first, no split once there is a CTA per SM.
-// The constants were fitted to an earlier form of the int8 kernel, whose position tile took a seventh longer, and serve
-// the f16-QK kernel too, whose tile takes two thirds of the present one. Checked with the present kernels against forced
-// pieces on ten shapes (16 to 2,048 tokens behind 100 to 148,000; the times above are of the int8 kernel): the choice is
-// within 2 % of the best for the int8 kernel; the f16-QK kernel on 50 tokens behind 3,000 takes 37.5 us and 36.5 with 10
-// pieces instead of 12, on an f16 cache 36.5 and 35.0, elsewhere within 2 % too.
-inline SplitPlan plan_prefill_rows(int M, int nkvh, int n_sm, int depth_hint, bool must_merge) {
-  constexpr double C0 = 3.0, CP = 4.0, M0 = 2.0, MROW = 1.2e-3, MPART = 2.0e-4;
+// The constants were fitted to an earlier form of the int8 kernel, whose position tile took a seventh longer. Checked with
+// the present kernels against forced pieces on fifty shapes (16 to 2,048 tokens behind 100 to 148,000; the times above are
+// of the int8 kernel): mostly within 2 % of the best. Known misses: up to some 150 tokens behind 200 to 800, left unsplit
+// where three pieces take 15 to 30 % less (16 behind 382, int8: 41.6 us and 31.2), and more than 48 pieces, which the
+// merge takes in two turns (39 of one KV head behind 9,071: 33.5 us with 55 pieces, 30.7 with 48).
+// f16_qk: the f16-QK kernel, whose position tile takes 1.0 to 1.2 us against 2.0: a merged row costs that many more tiles
+// (1,115 tokens of one KV head behind 2,906, 6,690 rows: 86 us unsplit on an f16 cache and 107 in two pieces, 100 and 113
+// with f16 Q K^T on a q8_0 cache; the int8 kernel 151 and 139. 600 of two KV heads behind 2,000, f16 cache: 66 and 101).
+inline SplitPlan plan_prefill_rows(int M, int nkvh, int n_sm, int depth_hint, bool must_merge, bool f16_qk) {
+  constexpr double C0 = 3.0, CP = 4.0, M0 = 2.0;
+  const double MROW = f16_qk ? 4.5e-3 : 1.2e-3, MPART = f16_qk ? 3.0e-4 : 2.0e-4;
   const int rt = row_tiles(M), ctas = rt * nkvh;
   SplitPlan plan;
   if (forced_plan(rt, must_merge, &plan)) return plan;
